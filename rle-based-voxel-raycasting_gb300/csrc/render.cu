@@ -345,6 +345,7 @@ __device__ __forceinline__ void draw_span(const Mask& mask, unsigned gmask, int 
                                           Counts& cnt) {
     const float u2dz = sp.u2dz, onedz2 = sp.onedz2;
     if constexpr (kCount) cnt.spans++;
+    __syncwarp(gmask);  // every lane has read the mask (horizon, y) before any lane claims
     const float mult = static_cast<float>(y + 1) - sp.scr_y1r;
     float uz = sp.u1z + u2dz * mult;
     float onez = sp.onez1 + onedz2 * mult;
@@ -1233,6 +1234,7 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             }
         }
     }
+    __syncwarp(gmask);  // every lane has read the mask before the group's next ray clears it
     if (kCount && active && k == 0) {
         // the lanes of a group hold the same counts; lane 0 adds the ray's
         unsigned long long* c = reinterpret_cast<unsigned long long*>(P.counters);

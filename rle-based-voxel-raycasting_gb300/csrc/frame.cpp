@@ -65,6 +65,7 @@ rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayPara
     p->nummaps = scene->nummaps;
     p->gridx0 = scene->lv[0].sx;
     p->gridz0 = scene->lv[0].sz;
+    while ((1 << p->log2x0) < p->gridx0) p->log2x0++;
     p->top_index = scene->top_index;
     p->height = scene->height;
     for (int m = 0; m < scene->nummaps; m++) {

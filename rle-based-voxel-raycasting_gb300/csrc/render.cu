@@ -39,6 +39,7 @@
 #include <cmath>
 #include <cstdint>
 
+#include "dda.h"
 #include "exact_steps.h"
 #include "rle_internal.h"
 
@@ -154,20 +155,13 @@ struct Ray {
     float ray_x, ray_z;
     float rmul;          // res_x2_mul_reverse (with the field-of-view focal length)
     float pos3d_z_add, pos3d_y_add;
-    float fix_x, fix_y;
+    int fix_x, fix_z;
     bool vertical;
     int ymin, ymax;      // clip range at the start (ymax < ymin: the ray is empty)
 };
 
 // Ray set-up: fan, 2D line, 3D direction, sample range, DDA start
 // (src/Cuda_Render.h:129-304).  Returns false if the ray covers no samples.
-struct Dda {
-    float g0x, g0y, g1x, g1y, gd0, gd1;
-    float i0x, i0y, i1x, i1y, dd0, dd1;
-    float dd_now, pnx, pny;
-    int index;
-};
-
 __device__ __forceinline__ bool setup_ray(const RayParams& P, int x, Ray& R, Dda& D) {
     const int S = P.S;
     const int r0 = P.res[0], r1 = P.res[1] + r0, r2 = P.res[2] + r1;
@@ -251,11 +245,11 @@ __device__ __forceinline__ bool setup_ray(const RayParams& P, int x, Ray& R, Dda
     const float dir_y = R.ray_x * P.sin_y - R.ray_z * P.cos_y;
     float sign_x = -1, sign_y = -1;
     R.fix_x = -1;
-    R.fix_y = -1;
+    R.fix_z = -1;
     float frac_x = P.posx - static_cast<float>(static_cast<int>(P.posx));
     float frac_y = P.posz - static_cast<float>(static_cast<int>(P.posz));
     if (dir_x >= 0) { R.fix_x = 0; sign_x = 1; frac_x = 1 - frac_x; }
-    if (dir_y >= 0) { R.fix_y = 0; sign_y = 1; frac_y = 1 - frac_y; }
+    if (dir_y >= 0) { R.fix_z = 0; sign_y = 1; frac_y = 1 - frac_y; }
     D.g0y = dir_y / fabsf(dir_x);
     D.g0x = sign_x;
     D.g1x = dir_x / fabsf(dir_y);
@@ -275,21 +269,26 @@ __device__ __forceinline__ bool setup_ray(const RayParams& P, int x, Ray& R, Dda
     return true;
 }
 
-// One DDA cell as the merge needs it.
+// One DDA cell: the distances along the ray where it begins and ends, its
+// column and the column's table entry.
 struct Cell {
-    float pz, py, czz, cyy;
-    uint32_t ex, ey;  // column-table entry
+    float near, far;
+    uint32_t ex, ey;
     int mip;
     int vx, vz;
-    bool loaded;
+    bool valid;
+};
+
+// A cell's projection: depth and screen numerator of its near edge at column
+// index 0, and what its far edge adds.
+struct Edge {
+    float pz, py, czz, cyy;
 };
 
 // Candidate runs a lane records per cell for the merge (shared memory, one
 // uint4 per run).  Six: since the scan drops runs whose samples are all
 // taken, cells rarely have more candidates.
 constexpr int kRecs = 6;
-// Samples of a span that one lane claims at a time: one word of bits.
-constexpr int kPiece = 32;
 
 // A lane's last coloured sample, stored one pass late: the colour gather
 // (a dependent load) then overlaps the following work instead of stalling
@@ -398,18 +397,11 @@ __device__ __forceinline__ void draw_span(const Mask& mask, unsigned gmask, int 
 // loop after the DDA step).  Uniform across the G lanes of the group.
 template <int G, bool kCount>
 __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, const Mask& mask, unsigned gmask, int k,
-                                           uint32_t* row, float* drow, rle_hit* hrow, Cell c, int& ymin, int& ymax,
-                                           Pending& pend, Counts& cnt) {
+                                           uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, const Edge& e, int& ymin,
+                                           int& ymax, Pending& pend, Counts& cnt) {
     const float res_y2 = static_cast<float>(P.S / 2);
     // clip top (:467)
-    if (c.pz * res_y2 + c.py <= c.pz * static_cast<float>(ymin)) return;
-    if (!c.loaded) {
-        const size_t ti = static_cast<size_t>(c.vx) + static_cast<size_t>(c.vz) * (P.gridx0 >> c.mip);
-        const uint2 e = in_bounds(ti < P.table_cols[c.mip], kBoundsTable, ti) ? __ldg(&P.table[c.mip][ti])
-                                                                               : make_uint2(0u, 0u);
-        c.ex = e.x;
-        c.ey = e.y;
-    }
+    if (e.pz * res_y2 + e.py <= e.pz * static_cast<float>(ymin)) return;
     if constexpr (kCount) cnt.fetched++;
     const uint16_t* hdr = P.slabs[c.mip] + 2 + c.ex;
     const int nruns = c.ey & 0xffffu;
@@ -434,15 +426,15 @@ __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, con
         sg += solid;
         const float sgf = static_cast<float>(sg);
         if constexpr (kCount) cnt.runs++;
-        float czz1 = c.pz, cyy1 = c.py;
-        if (mountain + sgs >= 0) { czz1 += c.czz; cyy1 += c.cyy; }
+        float czz1 = e.pz, cyy1 = e.py;
+        if (mountain + sgs >= 0) { czz1 += e.czz; cyy1 += e.cyy; }
         const float pz1 = czz1 + R.pos3d_z_add * sgs;
         if (pz1 <= 0) continue;
         const float py1 = cyy1 + R.pos3d_y_add * sgs;
         int scr_y2 = static_cast<int>(res_y2 + py1 / pz1);
         if (scr_y2 <= ymin) break;
-        float czz2 = c.pz, cyy2 = c.py;
-        if (mountain + sgf < 0) { czz2 += c.czz; cyy2 += c.cyy; }
+        float czz2 = e.pz, cyy2 = e.py;
+        if (mountain + sgf < 0) { czz2 += e.czz; cyy2 += e.cyy; }
         const float pz2 = czz2 + R.pos3d_z_add * sgf;
         if (pz2 <= 0) continue;
         const float py2 = cyy2 + R.pos3d_y_add * sgf;
@@ -460,7 +452,7 @@ __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, con
         }
         const int y = mask.first_clear(scr_y1, scr_y2);
         if (y >= scr_y2) continue;
-        const Span sp = span_setup(res_y2, R, c.pz, c.py, sgs, sgf, tex, texture);
+        const Span sp = span_setup(res_y2, R, e.pz, e.py, sgs, sgf, tex, texture);
         const uint64_t cofs = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(nruns);
         const uint64_t room = cofs <= P.slab_words[c.mip] ? P.slab_words[c.mip] - cofs : 0u;
         draw_span<G, kCount>(mask, gmask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, c.vx, c.vz,
@@ -471,45 +463,13 @@ __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, con
 
 // Where the DDA of one ray stands between chunks (uniform in its group).
 struct Walk {
-    Dda d;
+    Dda d;        // (dd_now, pnx, pny, index: the last event, right in the last lane at least)
+    DdaCache c;   // steps of d's chains, while `cached`
+    bool cached;
+    int room;     // steps that need no check for a LOD switch or the ray's end
     float z, dz, zswitch;
     int mapswitch, mip;
 };
-
-// One DDA step (:376-414), written with selects: the chain from one step to
-// the next is a compare and a select (the additions for both axes are issued
-// beside the compare), shorter than a branch on the compare.
-__device__ __forceinline__ void dda_step(Dda& d) {
-    const bool c1 = d.dd1 < d.dd0;
-    d.dd_now = c1 ? d.dd1 : d.dd0;
-    d.index = c1 ? 1 : 0;
-    d.pnx = c1 ? d.i1x : d.i0x;
-    d.pny = c1 ? d.i1y : d.i0y;
-    const float n1 = d.dd1 + d.gd1, n0 = d.dd0 + d.gd0;
-    const float a1x = d.i1x + d.g1x, a1y = d.i1y + d.g1y;
-    const float a0x = d.i0x + d.g0x, a0y = d.i0y + d.g0y;
-    d.dd1 = c1 ? n1 : d.dd1;
-    d.i1x = c1 ? a1x : d.i1x;
-    d.i1y = c1 ? a1y : d.i1y;
-    d.dd0 = c1 ? d.dd0 : n0;
-    d.i0x = c1 ? d.i0x : a0x;
-    d.i0y = c1 ? d.i0y : a0y;
-}
-
-// The update half of dda_step (c1: the step's compare): the state after the
-// step.  The step's own values (dd_now, pnx, pny, index) are selects on the
-// state before it, which dda_chunk forms only where a lane captures them.
-__device__ __forceinline__ void dda_advance(Dda& d, bool c1) {
-    const float n1 = d.dd1 + d.gd1, n0 = d.dd0 + d.gd0;
-    const float a1x = d.i1x + d.g1x, a1y = d.i1y + d.g1y;
-    const float a0x = d.i0x + d.g0x, a0y = d.i0y + d.g0y;
-    d.dd1 = c1 ? n1 : d.dd1;
-    d.i1x = c1 ? a1x : d.i1x;
-    d.i1y = c1 ? a1y : d.i1y;
-    d.dd0 = c1 ? d.dd0 : n0;
-    d.i0x = c1 ? d.i0x : a0x;
-    d.i0y = c1 ? d.i0y : a0y;
-}
 
 // Level-of-detail switch at the top of a step (:343-365): past the switch
 // distance the ray moves to the next mip level and doubles its step.
@@ -524,38 +484,22 @@ __device__ __forceinline__ void lod_switch(Walk& w, int nummaps) {
     }
 }
 
-// Derives the cell of one DDA step and, unless the horizon known now culls
-// it, starts the fetch of its column-table entry (the value is first used by
-// scan_runs, one chunk later in the pipeline).
-__device__ __forceinline__ void cell_geometry(const RayParams& P, const Ray& R, bool valid, float before, float delta,
-                                              float pbx, float pby, int ib, int mip, int ymin, Cell& c) {
-    const float res_y2 = static_cast<float>(P.S / 2);
-    const float sin_x = P.sin_x, cos_x = P.cos_x;
-    const float mountain = P.posy;
-    const int fxi = ib ? 0 : static_cast<int>(R.fix_x);
-    const int fzi = ib ? static_cast<int>(R.fix_y) : 0;
-    const float vs_x = R.ray_x * before;
-    const float vs_z = R.ray_z * before;
-    const int voxel_x = static_cast<int>(P.posx + pbx) + fxi;
-    const int voxel_z = static_cast<int>(P.posz + pby) + fzi;
+// Derives the column of one DDA step's cell and starts the fetch of its table
+// entry (the value is first used one chunk later in the pipeline).
+__device__ __forceinline__ void cell_fetch(const RayParams& P, const Ray& R, bool valid, float near, float far,
+                                           float pbx, float pby, int ib, int mip, Cell& c) {
+    const int voxel_x = static_cast<int>(P.posx + pbx) + (ib ? 0 : R.fix_x);
+    const int voxel_z = static_cast<int>(P.posz + pby) + (ib ? R.fix_z : 0);
+    c.near = near;
+    c.far = far;
     c.mip = mip;
-    c.vx = (voxel_x >> mip) & ((P.gridx0 >> mip) - 1);
-    c.vz = (voxel_z >> mip) & ((P.gridz0 >> mip) - 1);
-    const float corr_x = R.ray_x * delta;
-    const float corr_z = R.ray_z * delta;
-    c.pz = cos_x * vs_z + sin_x * mountain;
-    const float py = R.vertical ? cos_x * mountain - sin_x * vs_z : vs_x;
-    c.py = py * R.rmul;
-    c.czz = cos_x * corr_z;
-    const float cyy = R.vertical ? -sin_x * corr_z : corr_x;
-    c.cyy = cyy * R.rmul;
+    c.vx = (voxel_x & (P.gridx0 - 1)) >> mip;
+    c.vz = (voxel_z & (P.gridz0 - 1)) >> mip;
     c.ex = 0;
     c.ey = 0;
-    // clip top at the horizon known now; for pz >= 0 it only gets truer as ymin grows
-    const bool culled = c.pz >= 0.0f && c.pz * res_y2 + c.py <= c.pz * static_cast<float>(ymin);
-    c.loaded = valid && !culled;
-    if (c.loaded) {
-        const size_t ti = static_cast<size_t>(c.vx) + static_cast<size_t>(c.vz) * (P.gridx0 >> mip);
+    c.valid = valid;
+    if (valid) {
+        const uint32_t ti = static_cast<uint32_t>(c.vx) + (static_cast<uint32_t>(c.vz) << (P.log2x0 - mip));
         const uint2 e =
             in_bounds(ti < P.table_cols[mip], kBoundsTable, ti) ? __ldg(&P.table[mip][ti]) : make_uint2(0u, 0u);
         c.ex = e.x;
@@ -563,11 +507,28 @@ __device__ __forceinline__ void cell_geometry(const RayParams& P, const Ray& R, 
     }
 }
 
+__device__ __forceinline__ Edge cell_edge(const RayParams& P, const Ray& R, float near, float far) {
+    const float sin_x = P.sin_x, cos_x = P.cos_x;
+    const float mountain = P.posy;
+    const float delta = far - near;
+    const float vs_x = R.ray_x * near;
+    const float vs_z = R.ray_z * near;
+    const float corr_x = R.ray_x * delta;
+    const float corr_z = R.ray_z * delta;
+    Edge e;
+    e.pz = cos_x * vs_z + sin_x * mountain;
+    const float py = R.vertical ? cos_x * mountain - sin_x * vs_z : vs_x;
+    e.py = py * R.rmul;
+    e.czz = cos_x * corr_z;
+    const float cyy = R.vertical ? -sin_x * corr_z : corr_x;
+    e.cyy = cyy * R.rmul;
+    return e;
+}
+
 // Pre-culls a cell against the horizon at the start of its chunk and scans
 // its runs.  Returns the number of runs recorded in `rec` (one slot every
 // `stride` entries) that the exact walk could still draw, or -1 if the cell
-// has to be walked run by run at its turn; `pieces` is the number of
-// kPiece-sample pieces their spans make (1 for a cell to walk).
+// has to be walked run by run at its turn.
 //
 // A run is recorded unless, at the chunk's horizon, the walk would skip it for
 // good (`pz1 <= 0`, `pz2 <= 0`, `scr_y1 >= ymax`) or none of its samples in the
@@ -588,43 +549,46 @@ __device__ __forceinline__ void cell_geometry(const RayParams& P, const Ray& R, 
 //    the last horizon at which a recorded run still has a sample above it
 //    (for pz >= 0 it gets truer as ymin grows, for pz < 0 less true).
 __device__ __forceinline__ int scan_runs(const RayParams& P, const Ray& R, const Mask& mask, int ymin, int ymax,
-                                         const Cell& c, uint4* rec, int stride, int& pieces) {
+                                         const Cell& c, const Edge& e, uint4* rec, int stride) {
     const float res_y2 = static_cast<float>(P.S / 2);
     const float mountain = P.posy;
     const int mip = c.mip;
-    pieces = 0;
-    if (!c.loaded) return 0;
     // clip top at the current horizon
-    if (c.pz >= 0.0f && c.pz * res_y2 + c.py <= c.pz * static_cast<float>(ymin)) return 0;
+    if (e.pz >= 0.0f && e.pz * res_y2 + e.py <= e.pz * static_cast<float>(ymin)) return 0;
     const uint16_t* hdr = P.slabs[mip] + 2 + c.ex;
     const int nruns = c.ey & 0xffffu;
-    uint32_t sti = c.ey >> 16;
+    // headers are loaded two runs ahead: the first arrives with the table
+    // entry, and each later one would cost its latency in turn
+    auto header = [&](int r) -> uint32_t {
+        const uint64_t hi = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(r);
+        return r < nruns && in_bounds(hi < P.slab_words[mip], kBoundsHeader, hi) ? __ldg(&hdr[r]) : 0u;
+    };
+    uint32_t sti = c.ey >> 16, next = header(1), after = header(2);
     int sg = 0, texi = 0, n = 0;
     int low = 0x7fffffff;  // lowest reach (scr_y2) of the runs so far
     int top = 0;           // end of the highest recorded span
     for (int r = 0; r < nruns; r++) {
-        if (r > 0) {
-            const uint64_t hi = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(r);
-            sti = in_bounds(hi < P.slab_words[mip], kBoundsHeader, hi) ? __ldg(&hdr[r]) : 0u;
-        }
         const int solid = static_cast<int>(sti >> 10);
         sg += static_cast<int>(sti & 1023u) << mip;
+        sti = next;
+        next = after;
+        after = header(r + 3);
         if (solid == 0) continue;
         const int texture = texi, start = sg;
         texi += solid;
         const float sgs = static_cast<float>(sg);
         sg += solid << mip;
         const float sgf = static_cast<float>(sg);
-        float czz1 = c.pz, cyy1 = c.py;
-        if (mountain + sgs >= 0) { czz1 += c.czz; cyy1 += c.cyy; }
+        float czz1 = e.pz, cyy1 = e.py;
+        if (mountain + sgs >= 0) { czz1 += e.czz; cyy1 += e.cyy; }
         const float pz1 = czz1 + R.pos3d_z_add * sgs;
         if (pz1 <= 0) continue;
         const float py1 = cyy1 + R.pos3d_y_add * sgs;
         const int scr_y2 = static_cast<int>(res_y2 + py1 / pz1);
         if (scr_y2 <= ymin) break;  // the walk breaks here or earlier
         low = min(low, scr_y2);
-        float czz2 = c.pz, cyy2 = c.py;
-        if (mountain + sgf < 0) { czz2 += c.czz; cyy2 += c.cyy; }
+        float czz2 = e.pz, cyy2 = e.py;
+        if (mountain + sgf < 0) { czz2 += e.czz; cyy2 += e.cyy; }
         const float pz2 = czz2 + R.pos3d_z_add * sgf;
         if (pz2 <= 0) continue;
         const float py2 = cyy2 + R.pos3d_y_add * sgf;
@@ -633,29 +597,22 @@ __device__ __forceinline__ int scan_runs(const RayParams& P, const Ray& R, const
         const int hi = min(scr_y2, ymax);
         const int lo = mask.first_clear(max(scr_y1, ymin), hi);
         if (lo >= hi) continue;  // every sample it could colour is taken already
-        if (n == kRecs || scr_y2 != low) {
-            pieces = 1;
-            return -1;
-        }
+        if (n == kRecs || scr_y2 != low) return -1;
         rec[n * stride] = make_uint4(static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16),
                                      static_cast<uint32_t>(start),
                                      static_cast<uint32_t>(texture) | (static_cast<uint32_t>(solid) << 16), 0u);
         top = max(top, hi);
-        pieces += (hi - lo + kPiece - 1) / kPiece;
         n++;
     }
     if (n > 0) {
-        const int t = c.pz >= 0.0f ? top - 1 : ymin;
-        if (c.pz * res_y2 + c.py <= c.pz * static_cast<float>(t)) {
-            pieces = 1;
-            return -1;
-        }
+        const int t = e.pz >= 0.0f ? top - 1 : ymin;
+        if (e.pz * res_y2 + e.py <= e.pz * static_cast<float>(t)) return -1;
     }
     return n;
 }
 
 // Spans are not filled when their turn comes: their free samples are claimed
-// in the occupancy mask and queued in pieces of kPiece samples; a flush then
+// in the occupancy mask and queued in pieces, one per mask word; a flush then
 // colours the samples of up to G pieces G at a time, one sample per lane.
 // Queue entry: 2 x uint4 in shared memory, vector v of entry e at [v * G + e],
 //   {y0 | p0 << 14 | level << 28, claimed samples as bits from p0,
@@ -802,129 +759,106 @@ __device__ __forceinline__ uint32_t from_place(int n) {
     return r;
 }
 
+// The cell of lane `from`, and its projection, in every lane of the group.
+__device__ __forceinline__ Cell cell_of(unsigned gmask, const Cell& c, int from) {
+    Cell r;
+    r.near = r.far = 0.0f;  // in the projection
+    r.ex = __shfl_sync(gmask, c.ex, from);
+    r.ey = __shfl_sync(gmask, c.ey, from);
+    r.mip = __shfl_sync(gmask, c.mip, from);
+    r.vx = __shfl_sync(gmask, c.vx, from);
+    r.vz = __shfl_sync(gmask, c.vz, from);
+    r.valid = true;
+    return r;
+}
+__device__ __forceinline__ Edge edge_of(unsigned gmask, const Edge& e, int from) {
+    Edge r;
+    r.pz = __shfl_sync(gmask, e.pz, from);
+    r.py = __shfl_sync(gmask, e.py, from);
+    r.czz = __shfl_sync(gmask, e.czz, from);
+    r.cyy = __shfl_sync(gmask, e.cyy, from);
+    return r;
+}
+
 // Draws what the lanes' scans recorded, in the order of the sequential walk
-// (cell by cell, run by run), one piece of a span per lane: the chunk's
-// pieces are numbered in that order, G at a time go to the G lanes, and every
-// sample goes to the first span that covers it and finds it free.  For that
-// each lane takes its piece's window of the occupancy mask and removes the
-// spans before its own (their ranges come by shuffle).  A cell that has to be
-// walked is a barrier: the pieces before it are claimed first, then the group
-// walks it.
+// (cell by cell, run by run): every sample goes to the first span that covers
+// it and finds it free.  The chunk's records, numbered in that order, go one
+// to a lane; then, for each word of the occupancy mask that they reach, an OR
+// over the lanes before its own tells a lane which of its samples earlier
+// spans cover.  What is left of its span in the word, and free, it queues.  A
+// cell that has to be walked is a barrier: the records before it are claimed
+// first, then the group walks it.
 //
 // Bound by latency and issue: a frame ends with its slowest ray, and the
 // sequential form of this step (one record after another, two or three
 // dependent shared-memory loads and a queue insert each; spans of more than
-// 32 samples filled one at a time) took half of that ray.  Measured against
-// it, per frame: 1920x1080 466 -> 438 us, 3840x2160 (4096 samples) 424 -> 336
-// us, 1366x768 with hits 320 -> 278 us, 640x480 169 -> 152 us; a batch of 64
-// mixed frames at 16 lanes 7.34 -> 6.44 ms.
+// 32 samples filled one at a time) took half of that ray: 1920x1080 frames 466
+// -> 438 us and 3840x2160 frames 424 -> 336 us without it.  A prefix OR takes
+// five shuffles per word where one lane after another took 80 cycles per span
+// (4700 -> 3000 cycles per chunk that draws; 1920x1080 frames 350 -> 310 us).
 template <int G>
 __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, const Mask& mask, unsigned gmask, int k,
-                                            uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, int nrec,
-                                            int mine, const uint4* warp_recs, int stride, uint32_t* list, int& ymin,
+                                            uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, const Edge& edge,
+                                            int nrec, const uint4* warp_recs, int stride, uint32_t* list, int& ymin,
                                             int& ymax, Pending& pend, SpanQueue& q, Counts& cnt) {
     const int lb = lane_base(gmask);
-    if (!(__ballot_sync(gmask, mine != 0) & gmask)) return;
-    const bool multi = (__ballot_sync(gmask, mine > nrec && nrec > 0) & gmask) != 0u;  // some span has several pieces
-    // pieces before this lane's cell, and in all
-    int base, total;
-    if (!multi) {  // at most kRecs per lane: three bits
-        const unsigned n0 = __ballot_sync(gmask, mine & 1) & gmask, n1 = __ballot_sync(gmask, mine & 2) & gmask,
-                       n2 = __ballot_sync(gmask, mine & 4) & gmask;
-        const unsigned lt = (1u << (lb + k)) - 1u;
-        base = __popc(n0 & lt) + 2 * __popc(n1 & lt) + 4 * __popc(n2 & lt);
-        total = __popc(n0) + 2 * __popc(n1) + 4 * __popc(n2);
-    } else {
-        int incl = mine;
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) {
-            const int v = __shfl_up_sync(gmask, incl, o);
-            if (k >= o) incl += v;
-        }
-        base = incl - mine;
-        total = __shfl_sync(gmask, incl, lb + G - 1);
-    }
-    int carry = -1;  // first claimed sample of the span that runs over the last round's end
+    // entries before this lane's cell, and in all: its records (at most kRecs,
+    // three bits), or one for a cell to walk
+    const int mine = nrec < 0 ? 1 : nrec;
+    const unsigned n0 = __ballot_sync(gmask, mine & 1) & gmask, n1 = __ballot_sync(gmask, mine & 2) & gmask,
+                   n2 = __ballot_sync(gmask, mine & 4) & gmask;
+    const unsigned lt = (1u << (lb + k)) - 1u;
+    const int base = __popc(n0 & lt) + 2 * __popc(n1 & lt) + 4 * __popc(n2 & lt);
+    const int total = __popc(n0) + 2 * __popc(n1) + 4 * __popc(n2);
     for (int first = 0; first < total; first += G) {
         const int n = min(G, total - first);
-        // list[i] = lane | record << 5 | piece << 8 of entry i, or a cell to walk
-        if (nrec < 0) {
-            if (base >= first && base < first + G) list[base - first] = static_cast<uint32_t>(lb + k) | 0x80000000u;
-        } else if (!multi) {
-            for (int r = 0; r < nrec; r++) {
-                const int at = base + r - first;
-                if (at >= 0 && at < G) list[at] = static_cast<uint32_t>(lb + k) | (r << 5);
-            }
-        } else {
-            int at = base - first;
-            for (int r = 0; r < nrec && at < G; r++) {
-                const uint32_t range = warp_recs[r * stride + lb + k].x;
-                const int np = (static_cast<int>(range >> 16) - static_cast<int>(range & 0xffffu) + kPiece - 1) / kPiece;
-                for (int j = max(0, -at); j < np && at + j < G; j++)
-                    list[at + j] = static_cast<uint32_t>(lb + k) | (r << 5) | (j << 8);
-                at += np;
-            }
+        // list[i] = lane | record << 5 of entry i, or a cell to walk
+        for (int r = 0; r < mine; r++) {
+            const int at = base + r - first;
+            if (at >= 0 && at < G) list[at] = static_cast<uint32_t>(lb + k) | (r << 5) | (nrec < 0 ? 0x100u : 0u);
         }
         __syncwarp(gmask);  // the list and the records are read by the whole group
         const uint32_t entry = k < n ? list[k] : 0u;
         const int src = k < n ? static_cast<int>(entry & 31u) : lb;
-        const bool walk = (entry & 0x80000000u) != 0u;
+        const bool walk = (entry & 0x100u) != 0u;
         uint4 rec = make_uint4(0u, 0u, 0u, 0u);
         if (k < n && !walk) rec = warp_recs[static_cast<int>((entry >> 5) & 7u) * stride + src];
-        const uint32_t range = rec.x;  // of the whole span
-        const int piece = static_cast<int>((entry >> 8) & 0x3ffu);
-        const int lo = static_cast<int>(range & 0xffffu) + piece * kPiece;
-        const int hi = min(static_cast<int>(range >> 16), lo + kPiece);
-        const float pz = __shfl_sync(gmask, c.pz, src), py = __shfl_sync(gmask, c.py, src);
+        const int lo = static_cast<int>(rec.x & 0xffffu), hi = static_cast<int>(rec.x >> 16);
+        const float pz = __shfl_sync(gmask, edge.pz, src), py = __shfl_sync(gmask, edge.py, src);
         const int mip = __shfl_sync(gmask, c.mip, src);
         const uint32_t cofs = __shfl_sync(gmask, c.ex + 2u + (c.ey & 0xffffu), src);
         uint32_t vxz = 0;
         if (hrow) vxz = __shfl_sync(gmask, static_cast<uint32_t>(c.vx) | (static_cast<uint32_t>(c.vz) << 16), src);
         unsigned walks = (__ballot_sync(gmask, walk) & gmask) >> lb;
-        // the first lane of each span in this round, and of this lane's
-        const unsigned firsts =
-            (__ballot_sync(gmask, k < n && !walk && (piece == 0 || k == 0)) & gmask) >> lb;
-        const int head = 31 - __clz(static_cast<int>(firsts & (0xffffffffu >> (31 - k))) | 1);
         int start = 0;
         for (;;) {
             const int stop = walks ? __ffs(walks) - 1 : n;
             if (stop > start) {
                 // ---- spans [start, stop): claim the free samples ----
-                uint32_t own = 0;
-                const int wi = lo >> 5, sh = lo & 31;
-                if (k >= start && k < stop) {
-                    const uint32_t w0 = mask.w[wi], w1 = hi > 32 * wi + 32 ? mask.w[wi + 1] : 0u;
-                    own = ~__funnelshift_r(w0, w1, sh) & (0xffffffffu >> (32 - (hi - lo)));
-                }
-                // the spans before each lane's own (the last one is before none)
-                unsigned spans = (firsts >> start << start) & (0xffffffffu >> (32 - stop));
-                for (; spans & (spans - 1u); spans &= spans - 1u) {
-                    const int j = __ffs(spans) - 1;
-                    const uint32_t rj = __shfl_sync(gmask, range, lb + j);
-                    const uint32_t cover = from_place(static_cast<int>(rj & 0xffffu) - lo) &
-                                           ~from_place(static_cast<int>(rj >> 16) - lo);
-                    if (head > j) own &= ~cover;
-                }
-                const unsigned claims = (__ballot_sync(gmask, own != 0u) & gmask) >> lb;
-                if (claims) {
+                const bool in = k >= start && k < stop;
+                const int from = static_cast<int>(__reduce_min_sync(gmask, in ? static_cast<unsigned>(lo) : ~0u)) & ~31;
+                const int to = static_cast<int>(__reduce_max_sync(gmask, in ? static_cast<unsigned>(hi) : 0u));
+                int y0 = -1;  // the span's first claimed sample
+                for (int w = from; w < to; w += 32) {
+                    const uint32_t taken = mask.w[w >> 5];
+                    if (taken == 0xffffffffu) continue;
+                    const uint32_t bits = in ? from_place(lo - w) & ~from_place(hi - w) : 0u;
+                    uint32_t before = __shfl_up_sync(gmask, bits, 1);
+                    if (k == 0) before = 0u;
+#pragma unroll
+                    for (int o = 1; o < G; o <<= 1) {
+                        const uint32_t v = __shfl_up_sync(gmask, before, o);
+                        if (k >= o) before |= v;
+                    }
+                    const uint32_t own = bits & ~before & ~taken;
+                    const unsigned claims = (__ballot_sync(gmask, own != 0u) & gmask) >> lb;
+                    if (!claims) continue;
+                    mask.w[w >> 5] = taken | __reduce_or_sync(gmask, bits);  // by every lane, the same word
                     const int m = __popc(claims);
                     if (q.n + m > G) flush_spans<G>(P, R, q, gmask, k, row, drow, hrow, pend);
-                    const int skip = __ffs(own) - 1, p0 = lo + skip;
-                    int y0 = p0;
-                    if (multi) {
-                        // the span's first claimed sample, in this round or the last
-                        const unsigned of_span = claims & (0xffffffffu << head);
-                        y0 = __shfl_sync(gmask, p0, lb + (of_span ? __ffs(of_span) - 1 : 0));
-                        const int piece0 = __shfl_sync(gmask, piece, lb);
-                        if (head == 0 && piece0 > 0 && carry >= 0) y0 = carry;
-                        const int y0_last = __shfl_sync(gmask, of_span ? y0 : -1, lb + n - 1);
-                        const bool same = __shfl_sync(gmask, head, lb + n - 1) == 0 && piece0 > 0;
-                        carry = y0_last >= 0 ? y0_last : (same ? carry : -1);
-                    }
                     if (own) {
-                        atomicOr(&mask.w[wi], own << sh);
-                        const uint32_t over = sh ? own >> (32 - sh) : 0u;
-                        if (over) atomicOr(&mask.w[wi + 1], over);
+                        const int skip = __ffs(own) - 1, p0 = w + skip;
+                        if (y0 < 0) y0 = p0;
                         uint4* e = q.e + q.n + __popc(claims & ((1u << k) - 1u));
                         e[0] = make_uint4(static_cast<uint32_t>(y0) | (static_cast<uint32_t>(p0) << 14) |
                                               (static_cast<uint32_t>(mip) << 28),
@@ -933,30 +867,18 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
                     }
                     q.n += m;
                     __syncwarp(gmask);
-                    ymin = mask.first_clear(ymin, max(ymin, ymax));
-                    if (__ballot_sync(gmask, own != 0u && hi >= ymax) & gmask) ymax = mask.last_clear(ymin, ymax);
-                } else if (multi) {
-                    const int piece0 = __shfl_sync(gmask, piece, lb);
-                    if (!(__shfl_sync(gmask, head, lb + n - 1) == 0 && piece0 > 0)) carry = -1;
                 }
+                __syncwarp(gmask);  // the mask's words
+                ymin = mask.first_clear(ymin, max(ymin, ymax));
+                if (to >= ymax) ymax = mask.last_clear(ymin, ymax);
             }
             if (stop >= n || ymin >= ymax) break;
             // ---- a cell to walk ----
             walks &= walks - 1;
             start = stop + 1;
             const int from = __shfl_sync(gmask, src, lb + stop);
-            Cell cs;
-            cs.pz = __shfl_sync(gmask, c.pz, from);
-            cs.py = __shfl_sync(gmask, c.py, from);
-            cs.czz = __shfl_sync(gmask, c.czz, from);
-            cs.cyy = __shfl_sync(gmask, c.cyy, from);
-            cs.ex = __shfl_sync(gmask, c.ex, from);
-            cs.ey = __shfl_sync(gmask, c.ey, from);
-            cs.mip = __shfl_sync(gmask, c.mip, from);
-            cs.vx = __shfl_sync(gmask, c.vx, from);
-            cs.vz = __shfl_sync(gmask, c.vz, from);
-            cs.loaded = true;
-            merge_cell<G, false>(P, R, mask, gmask, k, row, drow, hrow, cs, ymin, ymax, pend, cnt);
+            merge_cell<G, false>(P, R, mask, gmask, k, row, drow, hrow, cell_of(gmask, c, from),
+                                 edge_of(gmask, edge, from), ymin, ymax, pend, cnt);
             if (start >= n || ymin >= ymax) break;
         }
         __syncwarp(gmask);  // the list and the records are rewritten
@@ -964,101 +886,173 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
     }
 }
 
-// One chunk of the DDA: G steps in lockstep, lane k keeping the state after
-// step k; the state before step k is the state after step k-1 (a shuffle
-// from lane k-1; lane 0 takes the chunk start).  Advances W past the chunk
-// and returns how many of its steps are valid (fewer than G: the ray ends).
+// One chunk of the DDA: lane k's cell is that of step k, from the event of
+// step k and that of the step before (a shuffle from lane k-1; lane 0 takes
+// the last event of the chunk before).  Advances W past the chunk and returns
+// how many of its steps are valid (fewer than G: the ray ends).
+//
+// Lane k finds the event of step k without the k steps before it (dda_jump).
+// Usually all lanes do, and the chunk is one straight line with the chains'
+// steps kept from the chunk before.  Where a chain leaves its binade, the
+// lanes up to there are done, the state goes one plain step on and the rest
+// jump again; a chain leaves its binade when the distance doubles, which is
+// one chunk in three (of 30) to one in seven (of 200).  LOD switches and the
+// ray's end cut a chunk the same way.  The ray's first chunk, where distances
+// double most, takes plain steps.
+//
+// Bound by latency and issue: in lockstep, G steps of 22 instructions each,
+// repeated by every lane, were 700 of a chunk's 860 instructions.  Together
+// with the horizon test that drops whole chunks before they are projected
+// (cell_alive) and the word-wise merge, per frame: 1920x1080 438 -> 310 us,
+// 1366x768 with hits 278 -> 225 us, 640x480 152 -> 130 us, 320x240 87 -> 82 us.
 struct ChunkStep {
-    float before, delta, pbx, pby;
+    float near, far, pbx, pby;
     int ib, mip;
 };
 
+// Steps from here that can meet neither a LOD switch nor the end of the ray.
+// z, dz (a power of two) and the switch distances are whole numbers held in
+// floats, exactly below 2^24.
+__device__ __forceinline__ int steps_unchecked(const RayParams& P, const Walk& W) {
+    if (!dda_can_jump(W.d) || !(W.z + W.dz < 16777216.0f)) return 0;
+    const int zi = static_cast<int>(W.z), shift = 31 - __clz(static_cast<int>(W.dz));
+    const int to_switch = W.mapswitch - zi, to_end = min(P.z_far, 16777216) - zi;
+    return to_switch < 0 || to_end < 0 ? 0 : min((to_switch >> shift) + 1, to_end >> shift);
+}
+
 template <int G>
 __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, unsigned gmask, ChunkStep& st) {
-    const float zfar = static_cast<float>(P.z_far);
-    // ---- 1. G DDA steps in lockstep; lane k keeps the state after step k ----
-    // the state before step k is the state after step k-1 (a shuffle
-    // from lane k-1; lane 0 takes the chunk start)
+    const int lb = lane_base(gmask);
     const float start_dd = W.d.dd_now, start_px = W.d.pnx, start_py = W.d.pny;
     const int start_ix = W.d.index;
     float c_dd = 0, c_px = 0, c_py = 0;
     int c_ix = 0, smip = W.mip;
     int nvalid = G;
-    // z, dz and the switch distances are integers held exactly in
-    // floats: when neither a LOD switch nor the end of the ray can
-    // fall inside the chunk, the steps need no checks
-    const int zi = static_cast<int>(W.z), dzi = static_cast<int>(W.dz);
-    // every step's z stays at or below the switch distance and the chunk's
-    // last z at or below z_far (dz > 0; the products stay far below 2^31)
-    const bool plain = W.mapswitch - zi >= (G - 1) * dzi && P.z_far - zi >= G * dzi;
-    if (plain) {
-#pragma unroll
-        for (int s = 0; s < G; s++) {
-            if (s == G - 1) {
+    bool done = false;
+    if (W.cached && W.room >= G) {
+        const DdaJump j = dda_jump(W.d, W.c, static_cast<float>(k));
+        const unsigned bad = __ballot_sync(gmask, !j.ok) & gmask;
+        const unsigned kept = __ballot_sync(gmask, j.kept);
+        const int src = lb + G - 1;
+        const float dd0 = __shfl_sync(gmask, j.dd0, src), dd1 = __shfl_sync(gmask, j.dd1, src);
+        const float i0x = __shfl_sync(gmask, j.i0x, src), i0y = __shfl_sync(gmask, j.i0y, src);
+        const float i1x = __shfl_sync(gmask, j.i1x, src), i1y = __shfl_sync(gmask, j.i1y, src);
+        c_dd = j.dd;
+        c_px = j.px;
+        c_py = j.py;
+        c_ix = j.axis1 ? 1 : 0;
+        done = bad == 0u;
+        if (done) {
+            W.d.dd0 = dd0;
+            W.d.dd1 = dd1;
+            W.d.i0x = i0x;
+            W.d.i0y = i0y;
+            W.d.i1x = i1x;
+            W.d.i1y = i1y;
+            W.cached = (kept >> src) & 1u;
+            W.z += W.dz * static_cast<float>(G);
+            W.room -= G;
+        }
+    }
+    if (!done) {
+        const float zfar = static_cast<float>(P.z_far);
+        int jumps = W.z == 0.0f ? 0 : 3;
+        int pos = 0;  // steps taken
+#pragma unroll 1
+        while (pos < G) {
+            const int lim = min(G, pos + W.room);
+            if (W.room > 0 && jumps > 0) {
+                jumps--;
+                if (!W.cached) W.c = dda_cache(W.d);
+                const DdaJump j = dda_jump(W.d, W.c, static_cast<float>(max(k - pos, 0)));
+                const unsigned bad = (__ballot_sync(gmask, k >= pos && !j.ok) & gmask) >> lb;
+                const unsigned kept = __ballot_sync(gmask, j.kept) >> lb;
+                const int stop = min(bad ? __ffs(bad) - 1 : G, lim);
+                if (k >= pos && k <= stop && k < lim) {
+                    c_dd = j.dd;
+                    c_px = j.px;
+                    c_py = j.py;
+                    c_ix = j.axis1 ? 1 : 0;
+                }
+                W.cached = true;
+                if (stop > pos) {
+                    const int src = lb + stop - 1;
+                    W.d.dd0 = __shfl_sync(gmask, j.dd0, src);
+                    W.d.i0x = __shfl_sync(gmask, j.i0x, src);
+                    W.d.i0y = __shfl_sync(gmask, j.i0y, src);
+                    W.d.dd1 = __shfl_sync(gmask, j.dd1, src);
+                    W.d.i1x = __shfl_sync(gmask, j.i1x, src);
+                    W.d.i1y = __shfl_sync(gmask, j.i1y, src);
+                    W.cached = (kept >> (stop - 1)) & 1u;
+                }
+                int taken = stop - pos;
+                if (stop < lim) {
+                    dda_step(W.d);
+                    W.cached = false;
+                    taken++;
+                }
+                W.z += W.dz * static_cast<float>(taken);
+                W.room -= taken;
+                pos += taken;
+            } else if (W.room > 0) {
+                W.z += W.dz * static_cast<float>(lim - pos);
+                W.room -= lim - pos;
+                W.cached = false;
+#pragma unroll 1
+                for (; pos < lim; pos++) {
+                    dda_step(W.d);
+                    if (pos == k) {
+                        c_dd = W.d.dd_now;
+                        c_px = W.d.pnx;
+                        c_py = W.d.pny;
+                        c_ix = W.d.index;
+                    }
+                }
+            } else {
+                if (W.z > W.zswitch) {
+                    lod_switch(W, P.nummaps);
+                    if (k >= pos) smip = W.mip;  // cells from this step on use the new level
+                }
+                W.z += W.dz;
+                if (W.z > zfar) {
+                    nvalid = pos;
+                    break;
+                }
                 dda_step(W.d);
-                if (s == k) {
+                if (pos == k) {
                     c_dd = W.d.dd_now;
                     c_px = W.d.pnx;
                     c_py = W.d.pny;
                     c_ix = W.d.index;
                 }
-            } else {
-                const bool c1 = W.d.dd1 < W.d.dd0;
-                if (s == k) {
-                    c_dd = c1 ? W.d.dd1 : W.d.dd0;
-                    c_px = c1 ? W.d.i1x : W.d.i0x;
-                    c_py = c1 ? W.d.i1y : W.d.i0y;
-                    c_ix = c1 ? 1 : 0;
-                }
-                dda_advance(W.d, c1);
+                pos++;
+                W.cached = false;
+                W.room = steps_unchecked(P, W);
             }
         }
-        W.z += W.dz * static_cast<float>(G);
-    } else {
-        bool ended_here = false;
-#pragma unroll 1
-        for (int s = 0; s < G; s++) {
-            if (W.z > W.zswitch) {
-                lod_switch(W, P.nummaps);
-                if (k >= s) smip = W.mip;  // cells from step s on use the new level
-            }
-            W.z += W.dz;
-            if (W.z > zfar) {
-                nvalid = s;
-                ended_here = true;
-                break;
-            }
-            dda_step(W.d);
-            if (s == k) {
-                c_dd = W.d.dd_now;
-                c_px = W.d.pnx;
-                c_py = W.d.pny;
-                c_ix = W.d.index;
-            }
-        }
-        (void)ended_here;
     }
-    float before = __shfl_up_sync(gmask, c_dd, 1);
-    float pbx = __shfl_up_sync(gmask, c_px, 1);
-    float pby = __shfl_up_sync(gmask, c_py, 1);
-    int ib = __shfl_up_sync(gmask, c_ix, 1);
-    if (k == 0) {
-        before = start_dd;
-        pbx = start_px;
-        pby = start_py;
-        ib = start_ix;
+    // the last event, for the next chunk's first cell
+    if (k == G - 1) {
+        W.d.dd_now = c_dd;
+        W.d.pnx = c_px;
+        W.d.pny = c_py;
+        W.d.index = c_ix;
     }
-    const float delta = c_dd - before;
-    st.before = before;
-    st.delta = delta;
-    st.pbx = pbx;
-    st.pby = pby;
-    st.ib = ib;
+    // lane k takes lane k-1's values and lane 0 those that the last lane had
+    // at the start of the chunk
+    const int prev = lb + (k + G - 1) % G;
+    const bool last = k == G - 1;
+    st.near = __shfl_sync(gmask, last ? start_dd : c_dd, prev);
+    st.pbx = __shfl_sync(gmask, last ? start_px : c_px, prev);
+    st.pby = __shfl_sync(gmask, last ? start_py : c_py, prev);
+    st.ib = __shfl_sync(gmask, last ? start_ix : c_ix, prev);
+    st.far = c_dd;
     st.mip = smip;
     return nvalid;
 }
 
-// Whether no cell at or beyond DDA distance t0 can draw a span.
+// What can still be drawn above the horizon ymin, as a bound that a cell is
+// tested against before anything of it is projected.
 //
 // A run whose top lies h below the eye (h = position.y + its column index,
 // level-0 units, h grows downwards) seen at distance t projects with
@@ -1066,25 +1060,44 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, uns
 // py_t = -rmul*sin_x*ray_z, py_h = rmul*cos_x for rays of the up/down fans,
 // py_t = rmul*ray_x, py_h = 0 for the left/right fans; :483-559).  The run is
 // dropped at its turn (`scr_y2 <= ymin`, or `pz1 <= 0`) whenever
-// f = K*pz1 + py1 < 0 with K = res_y2 - ymin - 1.  f is linear in (t, h), so
-// it stays negative for every t >= t0 and every h >= h0 (h0: the scene's
-// topmost voxel) if its slopes in t and h are not positive and f(t0, h0) < 0.
-// A margin of 1e-4 of the magnitudes of the terms covers the float rounding
-// of the kernel's evaluation (about 1e-6 relative); ymin only grows later,
-// which only lowers f where pz1 > 0.
-__device__ __forceinline__ bool ray_is_done(const RayParams& P, const Ray& R, float t0, int ymin) {
+// f = K*pz1 + py1 < 0 with K = res_y2 - ymin - 1.  f = a*t + b*h is linear, so
+// where its slope in h is not positive, f < 0 at a column's topmost run and at
+// the end of the cell where f is larger drops all of the column; and where
+// its slope in t is not positive either, f < 0 at the scene's topmost voxel
+// drops all cells from t on.  A margin of 1e-4 of the magnitudes of the terms
+// covers the float rounding of the kernel's evaluation (about 1e-6 relative);
+// ymin only grows later, which only lowers f where pz1 > 0.
+struct Horizon {
+    float a, b, eb;  // bound of f: a*t + b*h + eb*|h|
+    float scene;     // b*h + eb*|h| of the scene's topmost voxel, or +inf
+    int ymin;
+};
+
+__device__ __forceinline__ Horizon horizon_bound(const RayParams& P, const Ray& R, int ymin) {
     const float eps = 1e-4f;
     const float res_y2 = static_cast<float>(P.S / 2);
     const float K = res_y2 - static_cast<float>(ymin) - 1.0f;
     const float c = P.cos_x * R.ray_z, d = P.sin_x;
     const float py_t = R.vertical ? -R.rmul * P.sin_x * R.ray_z : R.rmul * R.ray_x;
     const float py_h = R.vertical ? R.rmul * P.cos_x : 0.0f;
-    const float a = K * c + py_t, b = K * d + py_h;
     const float scale = res_y2 + fabsf(K) + 1.0f;
     const float ma = fabsf(c) * scale + fabsf(py_t), mb = fabsf(d) * scale + fabsf(py_h);
     const float h0 = P.posy + static_cast<float>(P.top_index);
-    return a + eps * ma <= 0.0f && b + eps * mb <= 0.0f &&
-           a * t0 + b * h0 + eps * (ma * t0 + mb * fabsf(h0)) < 0.0f;
+    Horizon z;
+    z.a = K * c + py_t + eps * ma;
+    z.b = K * d + py_h;
+    z.eb = z.b + eps * mb <= 0.0f ? eps * mb : INFINITY;  // inf: the bound drops nothing
+    z.scene = z.a <= 0.0f ? z.b * h0 + z.eb * fabsf(h0) : INFINITY;
+    z.ymin = ymin;
+    return z;
+}
+
+// Whether the cell may draw: it has runs and the topmost is not below the
+// horizon for good.
+__device__ __forceinline__ bool cell_alive(const RayParams& P, const Horizon& z, const Cell& c) {
+    const float h = P.posy + static_cast<float>(static_cast<int>((c.ey >> 16) & 1023u) << c.mip);
+    const float bound = __fmaf_rn(z.a, z.a < 0.0f ? c.near : c.far, __fmaf_rn(z.b, h, z.eb * fabsf(h)));
+    return (c.ey & 0xffffu) != 0u && !(bound < 0.0f);
 }
 
 // Casts ray x of frame P with the G lanes of one group (lane k, lane mask
@@ -1147,19 +1160,16 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
                 W.dz *= 2;
             }
         }
+        W.cached = false;
+        W.room = W.z > W.zswitch ? 0 : steps_unchecked(P, W);
         ChunkStep st;
         int nvalid = dda_chunk<G>(P, W, k, gmask, st);
         Cell c;
-        cell_geometry(P, R, k < nvalid, st.before, st.delta, st.pbx, st.pby, st.ib, st.mip, ymin, c);
+        cell_fetch(P, R, k < nvalid, st.near, st.far, st.pbx, st.pby, st.ib, st.mip, c);
+        Horizon hz = horizon_bound(P, R, ymin);
         for (;;) {
             if (nvalid == 0) break;
             const bool ended = nvalid < G;
-            const bool valid = k < nvalid;
-            const float t_end = W.d.dd_now;  // DDA distance at the end of this chunk
-            // whether the ray can end after this chunk, tested at the horizon
-            // before the merge: ymin only grows, so a test that passes now
-            // passes after the merge too, and its latency hides under the DDA
-            const bool done_next = !kCount && ray_is_done(P, R, t_end, ymin);
             // ---- 1. the next chunk's DDA steps and column-table fetches are
             // issued now; their loads complete while this chunk is merged ----
             int nvalid_next = 0;
@@ -1167,51 +1177,50 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             if (!ended) {
                 ChunkStep st_next;
                 nvalid_next = dda_chunk<G>(P, W, k, gmask, st_next);
-                cell_geometry(P, R, k < nvalid_next, st_next.before, st_next.delta, st_next.pbx, st_next.pby,
-                              st_next.ib, st_next.mip, ymin, c_next);
+                cell_fetch(P, R, k < nvalid_next, st_next.near, st_next.far, st_next.pbx, st_next.pby, st_next.ib,
+                           st_next.mip, c_next);
             }
 
             if constexpr (kCount) {
                 // with counters every valid cell goes through the exact walk
-                unsigned todo = __ballot_sync(gmask, valid) >> lane_base(gmask);
+                const Edge edge = cell_edge(P, R, c.near, c.far);
+                unsigned todo = __ballot_sync(gmask, c.valid) >> lane_base(gmask);
                 if constexpr (G < 32) todo &= (1u << G) - 1u;
                 // the reference ends the ray when its horizon closes, checked
                 // at every step before the cell (:370)
                 for (; todo && ymin < ymax; todo &= todo - 1) {
                     const int src = lane_base(gmask) + __ffs(todo) - 1;
                     cnt.cells++;
-                    Cell cs;
-                    cs.pz = __shfl_sync(gmask, c.pz, src);
-                    cs.py = __shfl_sync(gmask, c.py, src);
-                    cs.czz = __shfl_sync(gmask, c.czz, src);
-                    cs.cyy = __shfl_sync(gmask, c.cyy, src);
-                    cs.ex = __shfl_sync(gmask, c.ex, src);
-                    cs.ey = __shfl_sync(gmask, c.ey, src);
-                    cs.mip = __shfl_sync(gmask, c.mip, src);
-                    cs.vx = __shfl_sync(gmask, c.vx, src);
-                    cs.vz = __shfl_sync(gmask, c.vz, src);
-                    cs.loaded = __shfl_sync(gmask, static_cast<int>(c.loaded), src) != 0;
-                    merge_cell<G, true>(P, R, mask, gmask, k, row, drow, hrow, cs, ymin, ymax, pend, cnt);
+                    merge_cell<G, true>(P, R, mask, gmask, k, row, drow, hrow, cell_of(gmask, c, src),
+                                        edge_of(gmask, edge, src), ymin, ymax, pend, cnt);
                 }
             } else {
-                // ---- 2. each lane: its cell -- pre-cull at the current horizon, run scan ----
-                int pieces;
-                const int nrec = scan_runs(P, R, mask, ymin, ymax, c, my_recs, blockDim.x, pieces);
-                // ---- 3. the recorded runs, in the order of the walk ----
-                merge_chunk<G>(P, R, mask, gmask, k, row, drow, hrow, c, nrec, pieces, warp_recs, blockDim.x, list,
-                               ymin, ymax, pend, q, cnt);
+                // ---- 2. each lane: its cell, unless it lies below the horizon ----
+                const bool alive = cell_alive(P, hz, c);
+                if (__ballot_sync(gmask, alive) & gmask) {
+                    const Edge edge = cell_edge(P, R, c.near, c.far);
+                    int nrec = 0;
+                    if (alive) nrec = scan_runs(P, R, mask, ymin, ymax, c, edge, my_recs, blockDim.x);
+                    // ---- 3. the recorded runs, in the order of the walk ----
+                    merge_chunk<G>(P, R, mask, gmask, k, row, drow, hrow, c, edge, nrec, warp_recs, blockDim.x, list,
+                                   ymin, ymax, pend, q, cnt);
+                    if (ymin != hz.ymin) hz = horizon_bound(P, R, ymin);
+                }
             }
             if (ymin >= ymax || ended) break;
             // Nothing further along this ray can be drawn once every run of
             // every later cell projects below the floating horizon (the
             // reference walks on to z_far without drawing).  Exact counters
             // need the full walk, so they keep it.
-            if (done_next) break;
+            if (!kCount) {
+                const float t_end = __shfl_sync(gmask, c.far, lane_base(gmask) + G - 1);
+                if (__fmaf_rn(hz.a, t_end, hz.scene) < 0.0f) break;
+            }
             // staging depth >= 2: the next chunk's table entries have arrived
             // under the merge; stage each cell's header line (second header
             // on; the first travels in the table entry) for its scan, which
             // follows the next DDA chunk
-            if (kStage && c_next.loaded && (c_next.ey & 0xffffu) > 1u)
+            if (kStage && c_next.valid && (c_next.ey & 0xffffu) > 1u)
                 stage_headers(P.slabs[c_next.mip] + 3 + c_next.ex, staging);
             c = c_next;
             nvalid = nvalid_next;

@@ -91,7 +91,8 @@ struct RayParams {
     int mapswitch0;               // MIP_DISTANCE * (0.25*(4-|rot.x|)), src/Cuda_Render.h:335
     int z_far;
     int nummaps;
-    int gridx0, gridz0;
+    int gridx0, gridz0;           // powers of two
+    int log2x0;                   // gridx0 = 1 << log2x0
     int top_index;                // scene's topmost voxel index (level-0 units)
     int height;                   // scene height (level 0)
     const uint2* table[RLE_MAX_MIPS];

@@ -1,8 +1,9 @@
-"""The closed forms of the fill's chains of float additions against the plain
-loops they stand for: the header the kernel includes, compiled for the host
-and compared bit for bit on random and on awkward inputs (ties, exact powers
-of two, sums that fall through binades or change sign, subnormals, infinities,
-NaN)."""
+"""The closed forms of the kernels' chains of float additions -- the fill's
+accumulators and the DDA's events -- against the plain loops they stand for:
+the header the kernels include, compiled for the host and compared bit for bit
+on random and on awkward inputs (ties, exact powers of two, sums that fall
+through binades or change sign, subnormals, infinities, NaN; rays along an
+axis to the last bit, eyes at negative coordinates, level switches)."""
 from __future__ import annotations
 
 import shutil
@@ -31,6 +32,6 @@ def check(tmp_path_factory):
 def test_closed_forms_equal_the_loops(check, seed):
     r = subprocess.run([str(check), str(seed), "400000"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
-    bad_acc, bad_steady, steady = map(int, r.stdout.split())
-    assert (bad_acc, bad_steady) == (0, 0)
-    assert steady > 50000  # the closed form is what was compared
+    bad_acc, bad_steady, bad_dda, steady, placed = map(int, r.stdout.split())
+    assert (bad_acc, bad_steady, bad_dda) == (0, 0, 0)
+    assert steady > 50000 and placed > 8000 * 60 * 32 // 2  # the closed form is what was compared

@@ -255,8 +255,10 @@ typedef struct rle_counters {
 } rle_counters;
 
 /* Launch shape of the raycast kernel (process-wide; 0 = built-in default).
- *   lanes_per_ray      lanes of a warp cooperating on one column ray: 8, 16
- *                      or 32 (4, 2 or 1 rays per warp); default 32
+ *   lanes_per_ray      8, 16 or 32; default 32.  Accepted, without effect on
+ *                      the launch: one warp of 32 lanes casts one column ray,
+ *                      which measured faster than 8 or 16 lanes per ray on
+ *                      every frame and batch
  *   cells_per_lane     DDA steps each lane takes per chunk: 1 (reserved)
  *   threads_per_block  32, 64, 96 or 128; default 128
  *   staging            staging depth of the column data a ray reads: 1 the
@@ -336,8 +338,8 @@ rle_status rle_render_frame(const rle_scene* scene, const rle_camera* cam,
  *     on the caller's stream, so up to eight frames are in flight and one
  *     frame's slowest column rays overlap the next frames';
  *   persistent: one raycast launch and one resolve launch for the whole
- *     batch -- the column rays of all frames form one work queue that lane
- *     groups drain tile by tile -- captured once (with the upload of the
+ *     batch -- the column rays of all frames form one work queue that warps
+ *     drain tile by tile -- captured once (with the upload of the
  *     per-frame parameters) into a CUDA graph and replayed for every batch.
  * rle_batch_autotune times both over its launch shapes.  No counterpart in
  * the reference, which renders one camera per launch
@@ -353,9 +355,9 @@ typedef struct rle_frame_request {
 } rle_frame_request;
 
 typedef struct rle_batch_tuning {
-    int tile_rays;          /* tile width: most adjacent column rays a lane group claims at
+    int tile_rays;          /* tile width: most adjacent column rays a warp claims at
                                once, 1..256 (default 1; claims shrink as the queue drains) */
-    int lanes_per_ray;      /* lanes cooperating on one column ray: 8, 16, 32 */
+    int lanes_per_ray;      /* 8, 16 or 32, as rle_tuning.lanes_per_ray */
     int staging;            /* staging depth of the column data, 1..3, as rle_tuning.staging */
     int threads_per_block;  /* 32, 64, 96 or 128 */
     int use_graph;          /* 1: capture once and replay (default); 0: plain launches */
@@ -381,11 +383,10 @@ size_t rle_batch_words_needed(const rle_frame_request* frames, int n);
  * the batch's ray buffer and parameter block), whatever streams they use. */
 rle_status rle_batch_render(rle_batch* b, const rle_scene* scene, const rle_frame_request* frames, int n,
                             void* stream);
-/* Times every tile_rays x lanes_per_ray x staging combination
- * ({1,2,4,8,16,32,64} x {8,16,32} x {1,2,3}: tile width, 4/2/1 rays per
- * warp, staging depth -- three independent axes) and the per-frame launches
- * (lanes {8,16,32} x staging {1,2,3}) on these frames (median of `repeats`
- * runs each), keeps the fastest as the batch's tuning and returns it. */
+/* Times every tile_rays x staging combination ({1,2,4,8,16,32,64} x {1,2,3}:
+ * tile width, staging depth) and the per-frame launches (staging {1,2,3}) on
+ * these frames (median of `repeats` runs each), keeps the fastest as the
+ * batch's tuning and returns it. */
 rle_status rle_batch_autotune(rle_batch* b, const rle_scene* scene, const rle_frame_request* frames, int n,
                               int repeats, rle_batch_tuning* best, float* best_ms);
 

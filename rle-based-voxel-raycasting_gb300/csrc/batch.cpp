@@ -121,7 +121,7 @@ void release(rle_batch* b) {
 }
 
 rle_status prepare_grid(rle_batch* b) {
-    rle_status st = rle::batch_grid_blocks(b->tuning.lanes_per_ray, b->tuning.threads_per_block, b->max_samples,
+    rle_status st = rle::batch_grid_blocks(b->tuning.threads_per_block, b->max_samples,
                                            b->with_hits, b->tuning.staging, &b->raycast_blocks);
     if (st != RLE_OK) return st;
     int sms = 0;
@@ -211,7 +211,6 @@ rle_status enqueue(rle_batch* b, int parity, cudaStream_t s) {
     rc.frames = reinterpret_cast<const rle::RayParams*>(b->d_params + L.ray_params);
     rc.tile = b->tuning.tile_rays;
     rc.staging = b->tuning.staging;
-    rc.lanes = b->tuning.lanes_per_ray;
     rc.threads = b->tuning.threads_per_block;
     rc.max_samples = b->max_samples;
     rc.blocks = b->raycast_blocks;
@@ -264,7 +263,6 @@ rle_status render_locked(rle_batch* b, const rle_scene* scene, const rle_scene* 
         for (int w = 0; w < k && e == cudaSuccess; w++) e = cudaStreamWaitEvent(b->workers[w], b->fork, 0);
         if (e != cudaSuccess) return cuda_fail(e, "rle_batch_render: fork to the worker streams");
         for (int i = 0; i < n && st == RLE_OK; i++) {
-            rp[i].lanes_per_ray = b->tuning.lanes_per_ray;
             rp[i].threads_per_block = b->tuning.threads_per_block;
             rp[i].staging = b->tuning.staging;
             st = rle::launch_raycast(rp[i], b->workers[i % k]);
@@ -474,37 +472,33 @@ extern "C" rle_status rle_batch_autotune(rle_batch* b, const rle_scene* scene, c
     rle_batch_tuning win = start;
     float win_ms = 1e30f;
     rle_status st = RLE_OK;
-    const int lanes[] = {8, 16, 32}, stagings[] = {1, 2, 3};
-    for (int lv : lanes) {
-        // the persistent launch over tile x staging, then the per-frame launches (tile -1)
-        for (int tv : {1, 2, 4, 8, 16, 32, 64, -1}) {
-            for (int sv : stagings) {
-                rle_batch_tuning t = start;
-                t.per_frame = tv < 0 ? 1 : 0;
-                t.tile_rays = tv < 0 ? start.tile_rays : tv;
-                t.lanes_per_ray = lv;
-                t.staging = sv;
-                if ((st = rle_batch_set_tuning(b, &t)) != RLE_OK) break;
-                if ((st = rle_batch_render(b, scene, frames, n, s)) != RLE_OK) break;  // warm-up / capture
-                std::vector<float> ms;
-                for (int r = 0; r < repeats && st == RLE_OK; r++) {
-                    cudaEventRecord(e0, s);
-                    st = rle_batch_render(b, scene, frames, n, s);
-                    cudaEventRecord(e1, s);
-                    cudaEventSynchronize(e1);
-                    float v = 0;
-                    cudaEventElapsedTime(&v, e0, e1);
-                    ms.push_back(v);
-                }
-                if (st != RLE_OK) break;
-                std::nth_element(ms.begin(), ms.begin() + ms.size() / 2, ms.end());
-                const float med = ms[ms.size() / 2];
-                if (med < win_ms) {
-                    win_ms = med;
-                    win = t;
-                }
+    // the persistent launch over tile x staging, then the per-frame launches (tile -1)
+    for (int tv : {1, 2, 4, 8, 16, 32, 64, -1}) {
+        for (int sv : {1, 2, 3}) {
+            rle_batch_tuning t = start;
+            t.per_frame = tv < 0 ? 1 : 0;
+            t.tile_rays = tv < 0 ? start.tile_rays : tv;
+            t.lanes_per_ray = 32;
+            t.staging = sv;
+            if ((st = rle_batch_set_tuning(b, &t)) != RLE_OK) break;
+            if ((st = rle_batch_render(b, scene, frames, n, s)) != RLE_OK) break;  // warm-up / capture
+            std::vector<float> ms;
+            for (int r = 0; r < repeats && st == RLE_OK; r++) {
+                cudaEventRecord(e0, s);
+                st = rle_batch_render(b, scene, frames, n, s);
+                cudaEventRecord(e1, s);
+                cudaEventSynchronize(e1);
+                float v = 0;
+                cudaEventElapsedTime(&v, e0, e1);
+                ms.push_back(v);
             }
             if (st != RLE_OK) break;
+            std::nth_element(ms.begin(), ms.begin() + ms.size() / 2, ms.end());
+            const float med = ms[ms.size() / 2];
+            if (med < win_ms) {
+                win_ms = med;
+                win = t;
+            }
         }
         if (st != RLE_OK) break;
     }

@@ -180,8 +180,6 @@ extern "C" rle_status rle_render_rays(const rle_scene* scene, const rle_raymap* 
     p.raydepth = d_raydepth;
     p.rayhit = d_rayhit;
     p.counters = d_counters;
-    p.lanes_per_ray = g_lanes_per_ray;
-    p.cells_per_lane = g_cells_per_lane;
     p.threads_per_block = g_threads_per_block;
     p.staging = g_staging;
     rle::DeviceGuard g(scene->device);
@@ -204,8 +202,6 @@ extern "C" rle_status rle_render_rays_timed(const rle_scene* scene, const rle_ra
     p.raybuf = d_raybuf;
     p.raydepth = d_raydepth;
     p.ray_time = d_times;
-    p.lanes_per_ray = g_lanes_per_ray;
-    p.cells_per_lane = g_cells_per_lane;
     p.threads_per_block = g_threads_per_block;
     p.staging = g_staging;
     rle::DeviceGuard g(scene->device);

@@ -8,19 +8,19 @@
 // perspective-correct colour and depth, culling with a floating horizon and
 // an occupancy bitmask.
 //
-// Parallel decomposition: a group of G lanes (G = 8, 16 or 32; 32/G rays
-// per warp) owns one ray.  The ray is processed in chunks of G DDA steps,
-// the next chunk's DDA and table fetches issued before this chunk's merge:
-//   1. all lanes step the DDA in lockstep (the DDA is a chain of IEEE
-//      additions, so every lane repeats the same operations) and lane k
-//      keeps the state of step k; the state before it comes from lane k-1;
-//   2. each lane, in parallel, derives its cell, pre-culls it against the
-//      horizon at the start of the chunk, fetches the column-table entry,
-//      scans the column's runs and records in shared memory the runs the
-//      walk could still draw;
+// Parallel decomposition: a warp owns one ray.  The ray is processed in chunks
+// of 32 DDA steps, the next chunk's DDA and table fetches issued before this
+// chunk's merge:
+//   1. lane k finds the state of step k of the DDA (a chain of IEEE additions
+//      per axis) without taking the steps before it, derives its cell and
+//      fetches the column-table entry; the state before it comes from lane
+//      k-1;
+//   2. each lane, in parallel, tests its cell against the horizon at the start
+//      of the chunk; where one passes, it scans its column's runs and records
+//      in shared memory the runs the walk could still draw;
 //   3. the recorded runs, in the order of the walk, go to the lanes, each of
 //      which claims the samples that its span covers first in the bitmask;
-//      the claimed samples are coloured later, G at a time.  Only a cell
+//      the claimed samples are coloured later, 32 at a time.  Only a cell
 //      whose outcome could depend on the horizon at its very turn is walked
 //      in sequence (scan_runs).
 // The pre-cull is conservative: the horizon only closes (ymin grows, ymax
@@ -117,8 +117,13 @@ __device__ __forceinline__ void stage_headers(const uint16_t* h, int staging) {
     else if (staging >= 3) asm volatile("prefetch.global.L1 [%0];" ::"l"(h));
 }
 
-// First lane of the group a lane mask describes.
-__device__ __forceinline__ int lane_base(unsigned gmask) { return __ffs(gmask) - 1; }
+// One warp owns one ray.  (Two or four rays per warp share its instructions
+// only while they take the same branches; the chunk that draws, the jump that
+// ends early and the ray that ends are branches.  Measured on batches, 8 / 16 /
+// 32 lanes per ray: 64 mixed frames 7.85 / 6.33 / 4.58 ms, eight 4K frames 3.25 /
+// 3.03 / 2.42 ms, 96 frames of 96x64 2.38 / 1.24 / 0.71 ms, persistent likewise.)
+constexpr int kLanes = 32;
+constexpr unsigned kWarp = 0xffffffffu;
 
 // Occupancy bitmask of one ray in shared memory (1 bit per sample).
 struct Mask {
@@ -292,7 +297,7 @@ constexpr int kRecs = 6;
 
 // A lane's last coloured sample, stored one pass late: the colour gather
 // (a dependent load) then overlaps the following work instead of stalling
-// the group at the store.  Every sample is written once, so the order of
+// the warp at the store.  Every sample is written once, so the order of
 // the stores does not matter.
 struct Pending {
     uint32_t* at = nullptr;
@@ -337,33 +342,33 @@ __device__ __forceinline__ Span span_setup(float res_y2, const Ray& R, float pz,
 }
 
 // Fills samples y .. scr_y2-1 of a span that the occupancy mask leaves open.
-template <int G, bool kCount>
-__device__ __forceinline__ void draw_span(const Mask& mask, unsigned gmask, int k, uint32_t* row, float* drow,
+template <bool kCount>
+__device__ __forceinline__ void draw_span(const Mask& mask, int k, uint32_t* row, float* drow,
                                           rle_hit* hrow, const uint16_t* colours, uint64_t colour_room, int S, int y,
                                           int scr_y2, const Span& sp, int mip, int vx, int vz, Pending& pend,
                                           Counts& cnt) {
     const float u2dz = sp.u2dz, onedz2 = sp.onedz2;
     if constexpr (kCount) cnt.spans++;
-    __syncwarp(gmask);  // every lane has read the mask (horizon, y) before any lane claims
+    __syncwarp();  // every lane has read the mask (horizon, y) before any lane claims
     const float mult = static_cast<float>(y + 1) - sp.scr_y1r;
     float uz = sp.u1z + u2dz * mult;
     float onez = sp.onez1 + onedz2 * mult;
     const float umin = static_cast<float>(sp.texture);
     const float umax = sp.umax;
-    // G pixels per pass: the accumulation runs in lockstep in every lane (it
+    // 32 pixels per pass: the accumulation runs in lockstep in every lane (it
     // is a chain of IEEE additions, one per sample, masked or not); lane k
     // keeps the values of sample y + k and does its divisions in parallel.
-    for (int y0 = y; y0 < scr_y2; y0 += G) {
-        const int n = min(G, scr_y2 - y0);
+    for (int y0 = y; y0 < scr_y2; y0 += kLanes) {
+        const int n = min(kLanes, scr_y2 - y0);
         // lane k needs the accumulators after k more additions
         float my_uz = uz, my_onez = onez;
         for (int j = 0; j < k && j < n; j++) {
             my_uz += u2dz;
             my_onez += onedz2;
         }
-        if (n == G) {  // start of the next pass: G additions from this one
-            uz = __shfl_sync(gmask, my_uz, (lane_base(gmask)) + G - 1) + u2dz;
-            onez = __shfl_sync(gmask, my_onez, (lane_base(gmask)) + G - 1) + onedz2;
+        if (n == kLanes) {  // start of the next pass: 32 additions from this one
+            uz = __shfl_sync(kWarp, my_uz, kLanes - 1) + u2dz;
+            onez = __shfl_sync(kWarp, my_onez, kLanes - 1) + onedz2;
         }
         const int yy = y0 + k;
         bool wrote = false;
@@ -388,15 +393,15 @@ __device__ __forceinline__ void draw_span(const Mask& mask, unsigned gmask, int 
             atomicOr(&mask.w[yy >> 5], 1u << (yy & 31));
             wrote = true;
         }
-        if constexpr (kCount) cnt.pixels += __popc(__ballot_sync(gmask, wrote));
-        __syncwarp(gmask);
+        if constexpr (kCount) cnt.pixels += __popc(__ballot_sync(kWarp, wrote));
+        __syncwarp();
     }
 }
 
 // Exact sequential processing of one cell (the body of the reference's main
-// loop after the DDA step).  Uniform across the G lanes of the group.
-template <int G, bool kCount>
-__device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, const Mask& mask, unsigned gmask, int k,
+// loop after the DDA step).  Uniform across the warp.
+template <bool kCount>
+__device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, const Mask& mask, int k,
                                            uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, const Edge& e, int& ymin,
                                            int& ymax, Pending& pend, Counts& cnt) {
     const float res_y2 = static_cast<float>(P.S / 2);
@@ -455,13 +460,13 @@ __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, con
         const Span sp = span_setup(res_y2, R, e.pz, e.py, sgs, sgf, tex, texture);
         const uint64_t cofs = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(nruns);
         const uint64_t room = cofs <= P.slab_words[c.mip] ? P.slab_words[c.mip] - cofs : 0u;
-        draw_span<G, kCount>(mask, gmask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, c.vx, c.vz,
+        draw_span<kCount>(mask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, c.vx, c.vz,
                              pend, cnt);
     }
 }
 
 
-// Where the DDA of one ray stands between chunks (uniform in its group).
+// Where the DDA of one ray stands between chunks (uniform in its warp).
 struct Walk {
     Dda d;        // (dd_now, pnx, pny, index: the last event, right in the last lane at least)
     DdaCache c;   // steps of d's chains, while `cached`
@@ -613,8 +618,8 @@ __device__ __forceinline__ int scan_runs(const RayParams& P, const Ray& R, const
 
 // Spans are not filled when their turn comes: their free samples are claimed
 // in the occupancy mask and queued in pieces, one per mask word; a flush then
-// colours the samples of up to G pieces G at a time, one sample per lane.
-// Queue entry: 2 x uint4 in shared memory, vector v of entry e at [v * G + e],
+// colours the samples of up to 32 pieces 32 at a time, one sample per lane.
+// Queue entry: 2 x uint4 in shared memory, vector v of entry e at [32 * v + e],
 //   {y0 | p0 << 14 | level << 28, claimed samples as bits from p0,
 //    colour offset of the column, texture | colours << 16},
 //   {pz, py, start of the run on the column axis, vx | vz << 16}
@@ -622,11 +627,11 @@ __device__ __forceinline__ int scan_runs(const RayParams& P, const Ray& R, const
 // p0 the piece's (sample indexes are below 2^14, a column holds fewer than
 // 2^16 colours and a run at most 63, so the fields fit).  The constants of
 // the fill (8 divisions) are formed by the lane that holds an entry in the
-// flush, for up to G pieces at once, and replace the second vector.
+// flush, for up to 32 pieces at once, and replace the second vector.
 constexpr int kQueueVecs = 2;
 
 struct SpanQueue {
-    uint4* e;  // G entries of this ray
+    uint4* e;  // 32 entries of this ray
     int n;
 };
 
@@ -646,25 +651,23 @@ __device__ __forceinline__ int nth_bit(uint32_t m, int r) {
     return at;
 }
 
-template <int G>
-__device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, SpanQueue& q, unsigned gmask, int k,
+__device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, SpanQueue& q, int k,
                                             uint32_t* row, float* drow, rle_hit* hrow, Pending& pend) {
     if (q.n == 0) return;
-    const int lb = lane_base(gmask);
     uint4 e0 = make_uint4(0u, 0u, 0u, 0u), e1 = e0;
     if (k < q.n) {
         e0 = q.e[k];
-        e1 = q.e[G + k];
+        e1 = q.e[kLanes + k];
     }
-    // samples per queued piece, inclusive prefix over the group's lanes
+    // samples per queued piece, inclusive prefix over the lanes
     const int cnt = __popc(e0.y);
     int incl = cnt;
 #pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-        const int v = __shfl_up_sync(gmask, incl, o);
+    for (int o = 1; o < kLanes; o <<= 1) {
+        const int v = __shfl_up_sync(kWarp, incl, o);
         if (k >= o) incl += v;
     }
-    const int total = __shfl_sync(gmask, incl, lb + q.n - 1);
+    const int total = __shfl_sync(kWarp, incl, q.n - 1);
     const int start = incl - cnt;
     // this lane's piece: the accumulators at its first sample and their step,
     // rounded (the sums are then one multiply-add away) or, where they leave
@@ -683,31 +686,30 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
         float du, dz;
         const bool jump = steady_step(uz, sp.u2dz, steps, &du) & steady_step(onez, sp.onedz2, steps, &dz);
         q.e[k].x = e0.x | (jump ? 0x80000000u : 0u);
-        q.e[G + k] = make_uint4(bits_of(uz), bits_of(jump ? du : sp.u2dz), bits_of(onez),
+        q.e[kLanes + k] = make_uint4(bits_of(uz), bits_of(jump ? du : sp.u2dz), bits_of(onez),
                                 bits_of(jump ? dz : sp.onedz2));
     }
-    __syncwarp(gmask);
-    for (int b = 0; b < total; b += G) {
+    __syncwarp();
+    for (int b = 0; b < total; b += kLanes) {
         const int t = b + k;
         // piece of sample t: entries start at strictly increasing sample
         // numbers (every queued piece owns at least one sample); those that
         // start at or before b, plus those starting in (b, b + k], count
         // the pieces at or before t
         const bool entry = k < q.n;
-        unsigned le = __ballot_sync(gmask, entry && start <= b) >> lb;
-        if constexpr (G < 32) le &= (1u << G) - 1u;
+        unsigned le = __ballot_sync(kWarp, entry && start <= b);
         const unsigned marks =
-            __reduce_or_sync(gmask, (entry && start > b && start < b + G) ? (1u << (start - b)) : 0u);
+            __reduce_or_sync(kWarp, (entry && start > b && start < b + kLanes) ? (1u << (start - b)) : 0u);
         const unsigned upto = k >= 31 ? 0xffffffffu : ((2u << k) - 1u);
-        const int from = lb + __popc(le) - 1 + __popc(marks & upto);
-        const int before = __shfl_sync(gmask, start, from);
+        const int from = __popc(le) - 1 + __popc(marks & upto);
+        const int before = __shfl_sync(kWarp, start, from);
         uint32_t vxz = 0, sg = 0;
         if (hrow) {
-            vxz = __shfl_sync(gmask, e1.w, from);
-            sg = __shfl_sync(gmask, e1.z, from);
+            vxz = __shfl_sync(kWarp, e1.w, from);
+            sg = __shfl_sync(kWarp, e1.z, from);
         }
         if (t < total) {
-            const uint4 v0 = q.e[from - lb], v1 = q.e[G + from - lb];
+            const uint4 v0 = q.e[from], v1 = q.e[kLanes + from];
             const uint32_t at = v0.x, cofs = v0.z, tc = v0.w;
             const int mip = static_cast<int>((at >> 28) & 7u);
             const int steps = nth_bit(v0.y, t - before);
@@ -747,7 +749,7 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
             }
         }
     }
-    __syncwarp(gmask);  // the entries are rewritten by the next spans
+    __syncwarp();  // the entries are rewritten by the next spans
     q.n = 0;
 }
 
@@ -759,24 +761,24 @@ __device__ __forceinline__ uint32_t from_place(int n) {
     return r;
 }
 
-// The cell of lane `from`, and its projection, in every lane of the group.
-__device__ __forceinline__ Cell cell_of(unsigned gmask, const Cell& c, int from) {
+// The cell of lane `from`, and its projection, in every lane.
+__device__ __forceinline__ Cell cell_of(const Cell& c, int from) {
     Cell r;
     r.near = r.far = 0.0f;  // in the projection
-    r.ex = __shfl_sync(gmask, c.ex, from);
-    r.ey = __shfl_sync(gmask, c.ey, from);
-    r.mip = __shfl_sync(gmask, c.mip, from);
-    r.vx = __shfl_sync(gmask, c.vx, from);
-    r.vz = __shfl_sync(gmask, c.vz, from);
+    r.ex = __shfl_sync(kWarp, c.ex, from);
+    r.ey = __shfl_sync(kWarp, c.ey, from);
+    r.mip = __shfl_sync(kWarp, c.mip, from);
+    r.vx = __shfl_sync(kWarp, c.vx, from);
+    r.vz = __shfl_sync(kWarp, c.vz, from);
     r.valid = true;
     return r;
 }
-__device__ __forceinline__ Edge edge_of(unsigned gmask, const Edge& e, int from) {
+__device__ __forceinline__ Edge edge_of(const Edge& e, int from) {
     Edge r;
-    r.pz = __shfl_sync(gmask, e.pz, from);
-    r.py = __shfl_sync(gmask, e.py, from);
-    r.czz = __shfl_sync(gmask, e.czz, from);
-    r.cyy = __shfl_sync(gmask, e.cyy, from);
+    r.pz = __shfl_sync(kWarp, e.pz, from);
+    r.py = __shfl_sync(kWarp, e.py, from);
+    r.czz = __shfl_sync(kWarp, e.czz, from);
+    r.cyy = __shfl_sync(kWarp, e.cyy, from);
     return r;
 }
 
@@ -787,7 +789,7 @@ __device__ __forceinline__ Edge edge_of(unsigned gmask, const Edge& e, int from)
 // over the lanes before its own tells a lane which of its samples earlier
 // spans cover.  What is left of its span in the word, and free, it queues.  A
 // cell that has to be walked is a barrier: the records before it are claimed
-// first, then the group walks it.
+// first, then the warp walks it.
 //
 // Bound by latency and issue: a frame ends with its slowest ray, and the
 // sequential form of this step (one record after another, two or three
@@ -796,66 +798,64 @@ __device__ __forceinline__ Edge edge_of(unsigned gmask, const Edge& e, int from)
 // -> 438 us and 3840x2160 frames 424 -> 336 us without it.  A prefix OR takes
 // five shuffles per word where one lane after another took 80 cycles per span
 // (4700 -> 3000 cycles per chunk that draws; 1920x1080 frames 350 -> 310 us).
-template <int G>
-__device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, const Mask& mask, unsigned gmask, int k,
+__device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, const Mask& mask, int k,
                                             uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, const Edge& edge,
                                             int nrec, const uint4* warp_recs, int stride, uint32_t* list, int& ymin,
                                             int& ymax, Pending& pend, SpanQueue& q, Counts& cnt) {
-    const int lb = lane_base(gmask);
     // entries before this lane's cell, and in all: its records (at most kRecs,
     // three bits), or one for a cell to walk
     const int mine = nrec < 0 ? 1 : nrec;
-    const unsigned n0 = __ballot_sync(gmask, mine & 1) & gmask, n1 = __ballot_sync(gmask, mine & 2) & gmask,
-                   n2 = __ballot_sync(gmask, mine & 4) & gmask;
-    const unsigned lt = (1u << (lb + k)) - 1u;
+    const unsigned n0 = __ballot_sync(kWarp, mine & 1), n1 = __ballot_sync(kWarp, mine & 2),
+                   n2 = __ballot_sync(kWarp, mine & 4);
+    const unsigned lt = (1u << k) - 1u;
     const int base = __popc(n0 & lt) + 2 * __popc(n1 & lt) + 4 * __popc(n2 & lt);
     const int total = __popc(n0) + 2 * __popc(n1) + 4 * __popc(n2);
-    for (int first = 0; first < total; first += G) {
-        const int n = min(G, total - first);
+    for (int first = 0; first < total; first += kLanes) {
+        const int n = min(kLanes, total - first);
         // list[i] = lane | record << 5 of entry i, or a cell to walk
         for (int r = 0; r < mine; r++) {
             const int at = base + r - first;
-            if (at >= 0 && at < G) list[at] = static_cast<uint32_t>(lb + k) | (r << 5) | (nrec < 0 ? 0x100u : 0u);
+            if (at >= 0 && at < kLanes) list[at] = static_cast<uint32_t>(k) | (r << 5) | (nrec < 0 ? 0x100u : 0u);
         }
-        __syncwarp(gmask);  // the list and the records are read by the whole group
+        __syncwarp();  // the list and the records are read by the whole warp
         const uint32_t entry = k < n ? list[k] : 0u;
-        const int src = k < n ? static_cast<int>(entry & 31u) : lb;
+        const int src = k < n ? static_cast<int>(entry & 31u) : 0;
         const bool walk = (entry & 0x100u) != 0u;
         uint4 rec = make_uint4(0u, 0u, 0u, 0u);
         if (k < n && !walk) rec = warp_recs[static_cast<int>((entry >> 5) & 7u) * stride + src];
         const int lo = static_cast<int>(rec.x & 0xffffu), hi = static_cast<int>(rec.x >> 16);
-        const float pz = __shfl_sync(gmask, edge.pz, src), py = __shfl_sync(gmask, edge.py, src);
-        const int mip = __shfl_sync(gmask, c.mip, src);
-        const uint32_t cofs = __shfl_sync(gmask, c.ex + 2u + (c.ey & 0xffffu), src);
+        const float pz = __shfl_sync(kWarp, edge.pz, src), py = __shfl_sync(kWarp, edge.py, src);
+        const int mip = __shfl_sync(kWarp, c.mip, src);
+        const uint32_t cofs = __shfl_sync(kWarp, c.ex + 2u + (c.ey & 0xffffu), src);
         uint32_t vxz = 0;
-        if (hrow) vxz = __shfl_sync(gmask, static_cast<uint32_t>(c.vx) | (static_cast<uint32_t>(c.vz) << 16), src);
-        unsigned walks = (__ballot_sync(gmask, walk) & gmask) >> lb;
+        if (hrow) vxz = __shfl_sync(kWarp, static_cast<uint32_t>(c.vx) | (static_cast<uint32_t>(c.vz) << 16), src);
+        unsigned walks = __ballot_sync(kWarp, walk);
         int start = 0;
         for (;;) {
             const int stop = walks ? __ffs(walks) - 1 : n;
             if (stop > start) {
                 // ---- spans [start, stop): claim the free samples ----
                 const bool in = k >= start && k < stop;
-                const int from = static_cast<int>(__reduce_min_sync(gmask, in ? static_cast<unsigned>(lo) : ~0u)) & ~31;
-                const int to = static_cast<int>(__reduce_max_sync(gmask, in ? static_cast<unsigned>(hi) : 0u));
+                const int from = static_cast<int>(__reduce_min_sync(kWarp, in ? static_cast<unsigned>(lo) : ~0u)) & ~31;
+                const int to = static_cast<int>(__reduce_max_sync(kWarp, in ? static_cast<unsigned>(hi) : 0u));
                 int y0 = -1;  // the span's first claimed sample
                 for (int w = from; w < to; w += 32) {
                     const uint32_t taken = mask.w[w >> 5];
                     if (taken == 0xffffffffu) continue;
                     const uint32_t bits = in ? from_place(lo - w) & ~from_place(hi - w) : 0u;
-                    uint32_t before = __shfl_up_sync(gmask, bits, 1);
+                    uint32_t before = __shfl_up_sync(kWarp, bits, 1);
                     if (k == 0) before = 0u;
 #pragma unroll
-                    for (int o = 1; o < G; o <<= 1) {
-                        const uint32_t v = __shfl_up_sync(gmask, before, o);
+                    for (int o = 1; o < kLanes; o <<= 1) {
+                        const uint32_t v = __shfl_up_sync(kWarp, before, o);
                         if (k >= o) before |= v;
                     }
                     const uint32_t own = bits & ~before & ~taken;
-                    const unsigned claims = (__ballot_sync(gmask, own != 0u) & gmask) >> lb;
+                    const unsigned claims = __ballot_sync(kWarp, own != 0u);
                     if (!claims) continue;
-                    mask.w[w >> 5] = taken | __reduce_or_sync(gmask, bits);  // by every lane, the same word
+                    mask.w[w >> 5] = taken | __reduce_or_sync(kWarp, bits);  // by every lane, the same word
                     const int m = __popc(claims);
-                    if (q.n + m > G) flush_spans<G>(P, R, q, gmask, k, row, drow, hrow, pend);
+                    if (q.n + m > kLanes) flush_spans(P, R, q, k, row, drow, hrow, pend);
                     if (own) {
                         const int skip = __ffs(own) - 1, p0 = w + skip;
                         if (y0 < 0) y0 = p0;
@@ -863,12 +863,12 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
                         e[0] = make_uint4(static_cast<uint32_t>(y0) | (static_cast<uint32_t>(p0) << 14) |
                                               (static_cast<uint32_t>(mip) << 28),
                                           own >> skip, cofs, rec.z);
-                        e[G] = make_uint4(__float_as_uint(pz), __float_as_uint(py), rec.y, vxz);
+                        e[kLanes] = make_uint4(__float_as_uint(pz), __float_as_uint(py), rec.y, vxz);
                     }
                     q.n += m;
-                    __syncwarp(gmask);
+                    __syncwarp();
                 }
-                __syncwarp(gmask);  // the mask's words
+                __syncwarp();  // the mask's words
                 ymin = mask.first_clear(ymin, max(ymin, ymax));
                 if (to >= ymax) ymax = mask.last_clear(ymin, ymax);
             }
@@ -876,12 +876,12 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
             // ---- a cell to walk ----
             walks &= walks - 1;
             start = stop + 1;
-            const int from = __shfl_sync(gmask, src, lb + stop);
-            merge_cell<G, false>(P, R, mask, gmask, k, row, drow, hrow, cell_of(gmask, c, from),
-                                 edge_of(gmask, edge, from), ymin, ymax, pend, cnt);
+            const int from = __shfl_sync(kWarp, src, stop);
+            merge_cell<false>(P, R, mask, k, row, drow, hrow, cell_of(c, from),
+                                 edge_of(edge, from), ymin, ymax, pend, cnt);
             if (start >= n || ymin >= ymax) break;
         }
-        __syncwarp(gmask);  // the list and the records are rewritten
+        __syncwarp();  // the list and the records are rewritten
         if (ymin >= ymax) return;
     }
 }
@@ -889,7 +889,7 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
 // One chunk of the DDA: lane k's cell is that of step k, from the event of
 // step k and that of the step before (a shuffle from lane k-1; lane 0 takes
 // the last event of the chunk before).  Advances W past the chunk and returns
-// how many of its steps are valid (fewer than G: the ray ends).
+// how many of its steps are valid (fewer than 32: the ray ends).
 //
 // Lane k finds the event of step k without the k steps before it (dda_jump).
 // Usually all lanes do, and the chunk is one straight line with the chains'
@@ -900,7 +900,7 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
 // ray's end cut a chunk the same way.  The ray's first chunk, where distances
 // double most, takes plain steps.
 //
-// Bound by latency and issue: in lockstep, G steps of 22 instructions each,
+// Bound by latency and issue: in lockstep, 32 steps of 22 instructions each,
 // repeated by every lane, were 700 of a chunk's 860 instructions.  Together
 // with the horizon test that drops whole chunks before they are projected
 // (cell_alive) and the word-wise merge, per frame: 1920x1080 438 -> 310 us,
@@ -920,23 +920,21 @@ __device__ __forceinline__ int steps_unchecked(const RayParams& P, const Walk& W
     return to_switch < 0 || to_end < 0 ? 0 : min((to_switch >> shift) + 1, to_end >> shift);
 }
 
-template <int G>
-__device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, unsigned gmask, ChunkStep& st) {
-    const int lb = lane_base(gmask);
+__device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, ChunkStep& st) {
     const float start_dd = W.d.dd_now, start_px = W.d.pnx, start_py = W.d.pny;
     const int start_ix = W.d.index;
     float c_dd = 0, c_px = 0, c_py = 0;
     int c_ix = 0, smip = W.mip;
-    int nvalid = G;
+    int nvalid = kLanes;
     bool done = false;
-    if (W.cached && W.room >= G) {
+    if (W.cached && W.room >= kLanes) {
         const DdaJump j = dda_jump(W.d, W.c, static_cast<float>(k));
-        const unsigned bad = __ballot_sync(gmask, !j.ok) & gmask;
-        const unsigned kept = __ballot_sync(gmask, j.kept);
-        const int src = lb + G - 1;
-        const float dd0 = __shfl_sync(gmask, j.dd0, src), dd1 = __shfl_sync(gmask, j.dd1, src);
-        const float i0x = __shfl_sync(gmask, j.i0x, src), i0y = __shfl_sync(gmask, j.i0y, src);
-        const float i1x = __shfl_sync(gmask, j.i1x, src), i1y = __shfl_sync(gmask, j.i1y, src);
+        const unsigned bad = __ballot_sync(kWarp, !j.ok);
+        const unsigned kept = __ballot_sync(kWarp, j.kept);
+        const int src = kLanes - 1;
+        const float dd0 = __shfl_sync(kWarp, j.dd0, src), dd1 = __shfl_sync(kWarp, j.dd1, src);
+        const float i0x = __shfl_sync(kWarp, j.i0x, src), i0y = __shfl_sync(kWarp, j.i0y, src);
+        const float i1x = __shfl_sync(kWarp, j.i1x, src), i1y = __shfl_sync(kWarp, j.i1y, src);
         c_dd = j.dd;
         c_px = j.px;
         c_py = j.py;
@@ -950,8 +948,8 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, uns
             W.d.i1x = i1x;
             W.d.i1y = i1y;
             W.cached = (kept >> src) & 1u;
-            W.z += W.dz * static_cast<float>(G);
-            W.room -= G;
+            W.z += W.dz * static_cast<float>(kLanes);
+            W.room -= kLanes;
         }
     }
     if (!done) {
@@ -959,15 +957,15 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, uns
         int jumps = W.z == 0.0f ? 0 : 3;
         int pos = 0;  // steps taken
 #pragma unroll 1
-        while (pos < G) {
-            const int lim = min(G, pos + W.room);
+        while (pos < kLanes) {
+            const int lim = min(kLanes, pos + W.room);
             if (W.room > 0 && jumps > 0) {
                 jumps--;
                 if (!W.cached) W.c = dda_cache(W.d);
                 const DdaJump j = dda_jump(W.d, W.c, static_cast<float>(max(k - pos, 0)));
-                const unsigned bad = (__ballot_sync(gmask, k >= pos && !j.ok) & gmask) >> lb;
-                const unsigned kept = __ballot_sync(gmask, j.kept) >> lb;
-                const int stop = min(bad ? __ffs(bad) - 1 : G, lim);
+                const unsigned bad = __ballot_sync(kWarp, k >= pos && !j.ok);
+                const unsigned kept = __ballot_sync(kWarp, j.kept);
+                const int stop = min(bad ? __ffs(bad) - 1 : kLanes, lim);
                 if (k >= pos && k <= stop && k < lim) {
                     c_dd = j.dd;
                     c_px = j.px;
@@ -976,13 +974,13 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, uns
                 }
                 W.cached = true;
                 if (stop > pos) {
-                    const int src = lb + stop - 1;
-                    W.d.dd0 = __shfl_sync(gmask, j.dd0, src);
-                    W.d.i0x = __shfl_sync(gmask, j.i0x, src);
-                    W.d.i0y = __shfl_sync(gmask, j.i0y, src);
-                    W.d.dd1 = __shfl_sync(gmask, j.dd1, src);
-                    W.d.i1x = __shfl_sync(gmask, j.i1x, src);
-                    W.d.i1y = __shfl_sync(gmask, j.i1y, src);
+                    const int src = stop - 1;
+                    W.d.dd0 = __shfl_sync(kWarp, j.dd0, src);
+                    W.d.i0x = __shfl_sync(kWarp, j.i0x, src);
+                    W.d.i0y = __shfl_sync(kWarp, j.i0y, src);
+                    W.d.dd1 = __shfl_sync(kWarp, j.dd1, src);
+                    W.d.i1x = __shfl_sync(kWarp, j.i1x, src);
+                    W.d.i1y = __shfl_sync(kWarp, j.i1y, src);
                     W.cached = (kept >> (stop - 1)) & 1u;
                 }
                 int taken = stop - pos;
@@ -1032,7 +1030,7 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, uns
         }
     }
     // the last event, for the next chunk's first cell
-    if (k == G - 1) {
+    if (k == kLanes - 1) {
         W.d.dd_now = c_dd;
         W.d.pnx = c_px;
         W.d.pny = c_py;
@@ -1040,12 +1038,12 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, uns
     }
     // lane k takes lane k-1's values and lane 0 those that the last lane had
     // at the start of the chunk
-    const int prev = lb + (k + G - 1) % G;
-    const bool last = k == G - 1;
-    st.near = __shfl_sync(gmask, last ? start_dd : c_dd, prev);
-    st.pbx = __shfl_sync(gmask, last ? start_px : c_px, prev);
-    st.pby = __shfl_sync(gmask, last ? start_py : c_py, prev);
-    st.ib = __shfl_sync(gmask, last ? start_ix : c_ix, prev);
+    const int prev = (k + kLanes - 1) % kLanes;
+    const bool last = k == kLanes - 1;
+    st.near = __shfl_sync(kWarp, last ? start_dd : c_dd, prev);
+    st.pbx = __shfl_sync(kWarp, last ? start_px : c_px, prev);
+    st.pby = __shfl_sync(kWarp, last ? start_py : c_py, prev);
+    st.ib = __shfl_sync(kWarp, last ? start_ix : c_ix, prev);
     st.far = c_dd;
     st.mip = smip;
     return nvalid;
@@ -1100,14 +1098,12 @@ __device__ __forceinline__ bool cell_alive(const RayParams& P, const Horizon& z,
     return (c.ey & 0xffffu) != 0u && !(bound < 0.0f);
 }
 
-// Casts ray x of frame P with the G lanes of one group (lane k, lane mask
-// gmask), using mask_words (S/32 words of shared memory) as its bitmask.
-// active = false: the lanes only take part in the group's collectives.
-// chunks of G DDA steps, lane k taking step k of each.
-template <int G, bool kCount, bool kHits, bool kStage>
+// Casts ray x of frame P with one warp (lane k), using mask_words (S/32 words
+// of shared memory) as its bitmask, in chunks of 32 DDA steps, lane k taking
+// step k of each.
+template <bool kCount, bool kHits, bool kStage>
 __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active, uint32_t* mask_words, uint4* recs,
-                                         uint4* spans, uint32_t* list, int k, unsigned gmask, int staging,
-                                         Counts& cnt) {
+                                         uint4* spans, uint32_t* list, int k, int staging, Counts& cnt) {
     const int S = P.S;
     const int words = (S + 31) >> 5;
     Mask mask{mask_words};
@@ -1120,18 +1116,12 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
     Walk W;
     bool live = false;
     if (active) {
-        for (int w = k; w < words; w += G) mask.w[w] = 0;
+        for (int w = k; w < words; w += kLanes) mask.w[w] = 0;
         live = setup_ray(P, x, R, W.d);
     } else {
         R.ymin = 0;
         R.ymax = -1;
     }
-    // A whole-warp barrier, also with several rays per warp: every lane that
-    // has not exited passes one at the start and one at the end of each ray
-    // (a group with no ray left exits, and exited lanes do not count), so it
-    // always completes -- and it brings a warp's groups back into step at
-    // their ray boundaries, where they then issue together (a barrier over
-    // the group alone measured 6% slower for 4K batches at 16 lanes).
     __syncwarp();
     uint32_t* row = active ? P.raybuf + static_cast<size_t>(x) * S : nullptr;
     float* drow = active ? P.raydepth + static_cast<size_t>(x) * S : nullptr;
@@ -1163,20 +1153,20 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
         W.cached = false;
         W.room = W.z > W.zswitch ? 0 : steps_unchecked(P, W);
         ChunkStep st;
-        int nvalid = dda_chunk<G>(P, W, k, gmask, st);
+        int nvalid = dda_chunk(P, W, k, st);
         Cell c;
         cell_fetch(P, R, k < nvalid, st.near, st.far, st.pbx, st.pby, st.ib, st.mip, c);
         Horizon hz = horizon_bound(P, R, ymin);
         for (;;) {
             if (nvalid == 0) break;
-            const bool ended = nvalid < G;
+            const bool ended = nvalid < kLanes;
             // ---- 1. the next chunk's DDA steps and column-table fetches are
             // issued now; their loads complete while this chunk is merged ----
             int nvalid_next = 0;
             Cell c_next;
             if (!ended) {
                 ChunkStep st_next;
-                nvalid_next = dda_chunk<G>(P, W, k, gmask, st_next);
+                nvalid_next = dda_chunk(P, W, k, st_next);
                 cell_fetch(P, R, k < nvalid_next, st_next.near, st_next.far, st_next.pbx, st_next.pby, st_next.ib,
                            st_next.mip, c_next);
             }
@@ -1184,25 +1174,24 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             if constexpr (kCount) {
                 // with counters every valid cell goes through the exact walk
                 const Edge edge = cell_edge(P, R, c.near, c.far);
-                unsigned todo = __ballot_sync(gmask, c.valid) >> lane_base(gmask);
-                if constexpr (G < 32) todo &= (1u << G) - 1u;
+                unsigned todo = __ballot_sync(kWarp, c.valid);
                 // the reference ends the ray when its horizon closes, checked
                 // at every step before the cell (:370)
                 for (; todo && ymin < ymax; todo &= todo - 1) {
-                    const int src = lane_base(gmask) + __ffs(todo) - 1;
+                    const int src = __ffs(todo) - 1;
                     cnt.cells++;
-                    merge_cell<G, true>(P, R, mask, gmask, k, row, drow, hrow, cell_of(gmask, c, src),
-                                        edge_of(gmask, edge, src), ymin, ymax, pend, cnt);
+                    merge_cell<true>(P, R, mask, k, row, drow, hrow, cell_of(c, src),
+                                        edge_of(edge, src), ymin, ymax, pend, cnt);
                 }
             } else {
                 // ---- 2. each lane: its cell, unless it lies below the horizon ----
                 const bool alive = cell_alive(P, hz, c);
-                if (__ballot_sync(gmask, alive) & gmask) {
+                if (__ballot_sync(kWarp, alive)) {
                     const Edge edge = cell_edge(P, R, c.near, c.far);
                     int nrec = 0;
                     if (alive) nrec = scan_runs(P, R, mask, ymin, ymax, c, edge, my_recs, blockDim.x);
                     // ---- 3. the recorded runs, in the order of the walk ----
-                    merge_chunk<G>(P, R, mask, gmask, k, row, drow, hrow, c, edge, nrec, warp_recs, blockDim.x, list,
+                    merge_chunk(P, R, mask, k, row, drow, hrow, c, edge, nrec, warp_recs, blockDim.x, list,
                                    ymin, ymax, pend, q, cnt);
                     if (ymin != hz.ymin) hz = horizon_bound(P, R, ymin);
                 }
@@ -1213,7 +1202,7 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             // reference walks on to z_far without drawing).  Exact counters
             // need the full walk, so they keep it.
             if (!kCount) {
-                const float t_end = __shfl_sync(gmask, c.far, lane_base(gmask) + G - 1);
+                const float t_end = __shfl_sync(kWarp, c.far, kLanes - 1);
                 if (__fmaf_rn(hz.a, t_end, hz.scene) < 0.0f) break;
             }
             // staging depth >= 2: the next chunk's table entries have arrived
@@ -1226,13 +1215,13 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             nvalid = nvalid_next;
         }
     }
-    flush_spans<G>(P, R, q, gmask, k, row, drow, hrow, pend);
+    flush_spans(P, R, q, k, row, drow, hrow, pend);
     pend.flush();
-    __syncwarp();  // whole warp, as at the start of the ray
+    __syncwarp();
 
     // ---- coalesced fill of the samples no span coloured ----
     if (active) {
-        for (int y = k; y < S; y += G) {
+        for (int y = k; y < S; y += kLanes) {
             if (mask.get(y)) continue;
             const bool in = y >= ymin0 && y <= ymax0;
             row[y] = in ? kSky : 0u;
@@ -1243,9 +1232,9 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             }
         }
     }
-    __syncwarp(gmask);  // every lane has read the mask before the group's next ray clears it
+    __syncwarp();  // every lane has read the mask before the warp's next ray clears it
     if (kCount && active && k == 0) {
-        // the lanes of a group hold the same counts; lane 0 adds the ray's
+        // the lanes hold the same counts; lane 0 adds the ray's
         unsigned long long* c = reinterpret_cast<unsigned long long*>(P.counters);
         const unsigned long long v[6] = {cnt.cells, cnt.fetched, cnt.headers, cnt.runs, cnt.spans, cnt.pixels};
         for (int i = 0; i < 6; i++)
@@ -1254,10 +1243,9 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
     cnt = Counts();
 }
 
-// Shared memory of a raycast block: the rays' occupancy masks (`words` per
-// ray slot, padded to 16 bytes), then per thread kRecs run records, the span
-// queues (one entry per lane of the group) and the merge's entry list (one
-// word per lane).
+// Shared memory of a raycast block: the warps' occupancy masks (`words` each,
+// padded to 16 bytes), then per thread kRecs run records, the span
+// queues (one entry per lane) and the merge's entry list (one word per lane).
 __host__ __device__ __forceinline__ int mask_region_words(int slots, int words) {
     return (slots * words + 3) & ~3;
 }
@@ -1266,54 +1254,41 @@ __host__ __device__ __forceinline__ size_t raycast_smem_bytes(int threads, int s
            static_cast<size_t>(threads) * (kRecs * sizeof(uint4) + kQueueVecs * sizeof(uint4) + sizeof(uint32_t));
 }
 struct BlockSmem {
+    int k, slots, slot;  // lane, warps of the block, this warp
+    uint32_t* mask;      // this warp's mask
     uint4* recs;
-    uint4* spans;    // this ray slot's queue
-    uint32_t* list;  // this ray slot's list
-    __device__ __forceinline__ BlockSmem(uint32_t* smem, int words, int slots, int slot, int lanes) {
+    uint4* spans;        // this warp's queue
+    uint32_t* list;      // this warp's list
+    __device__ __forceinline__ BlockSmem(uint32_t* smem, int words) {
+        k = threadIdx.x % kLanes;
+        slots = blockDim.x / kLanes;
+        slot = threadIdx.x / kLanes;
+        mask = smem + slot * words;
         recs = reinterpret_cast<uint4*>(smem + mask_region_words(slots, words));
         uint4* queues = recs + blockDim.x * kRecs;
-        spans = queues + slot * (kQueueVecs * lanes);
-        list = reinterpret_cast<uint32_t*>(queues + blockDim.x * kQueueVecs) + slot * lanes;
-    }
-};
-
-// Lane layout of a group of G lanes within a block.
-template <int G>
-struct Lanes {
-    int lane, g, k, slot;
-    unsigned gmask;
-    __device__ __forceinline__ Lanes() {
-        constexpr int kGroups = 32 / G;
-        lane = threadIdx.x & 31;
-        g = lane / G;  // ray group within the warp
-        k = lane % G;  // lane within the group
-        gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (g * G));
-        slot = (threadIdx.x >> 5) * kGroups + g;  // ray slot within the block
+        spans = queues + slot * (kQueueVecs * kLanes);
+        list = reinterpret_cast<uint32_t*>(queues + blockDim.x * kQueueVecs) + slot * kLanes;
     }
 };
 
 // One frame: ray slot s of block b casts ray b * slots + s.  kCount: the
 // DETAIL_BENCH counters (exact walk of every cell); kHits: hit records;
 // kStage: run-header staging (depth 2/3).
-template <int G, bool kCount, bool kHits, bool kStage>
+template <bool kCount, bool kHits, bool kStage>
 __global__ void __launch_bounds__(128, 4) raycast_kernel(const __grid_constant__ RayParams P) {
     extern __shared__ uint32_t smem[];
-    const Lanes<G> L;
-    const int rays_per_block = (blockDim.x >> 5) * (32 / G);
-    const int x = blockIdx.x * rays_per_block + L.slot;
-    const int words = (P.S + 31) >> 5;
-    const BlockSmem B(smem, words, rays_per_block, L.slot, G);
+    const BlockSmem B(smem, (P.S + 31) >> 5);
+    const int x = blockIdx.x * B.slots + B.slot;
     Counts cnt;
-    // per-ray timing (rle_render_rays_timed): the first lane of the group
+    // per-ray timing (rle_render_rays_timed): the first lane
     // stamps the ray's start and end; nothing else changes
-    if (P.ray_time && L.k == 0 && x < P.rays) {
+    if (P.ray_time && B.k == 0 && x < P.rays) {
         rle_ray_time* t = P.ray_time + x;
         t->start_ns = global_ns();
         t->start_clock = static_cast<uint64_t>(clock64());
     }
-    cast_ray<G, kCount, kHits, kStage>(P, x, x < P.rays, smem + L.slot * words, B.recs, B.spans, B.list, L.k, L.gmask,
-                                       P.staging, cnt);
-    if (P.ray_time && L.k == 0 && x < P.rays) {
+    cast_ray<kCount, kHits, kStage>(P, x, x < P.rays, B.mask, B.recs, B.spans, B.list, B.k, P.staging, cnt);
+    if (P.ray_time && B.k == 0 && x < P.rays) {
         rle_ray_time* t = P.ray_time + x;
         t->end_clock = static_cast<uint64_t>(clock64());
         t->end_ns = global_ns();
@@ -1323,35 +1298,33 @@ __global__ void __launch_bounds__(128, 4) raycast_kernel(const __grid_constant__
 }
 
 // Many frames in one persistent launch.  The rays of all frames form one
-// index space (ray_start[f] = first global ray of frame f); each group takes
+// index space (ray_start[f] = first global ray of frame f); each warp takes
 // `tile` consecutive rays at a time from a global counter until none are
 // left, so long and short rays of every frame balance across the GPU.
-template <int G, bool kHits, bool kStage>
+template <bool kHits, bool kStage>
 __global__ void __launch_bounds__(128, 4) raycast_batch_kernel(BatchHeader* hdr, const int* __restrict__ ray_start,
                                                             const RayParams* __restrict__ frames, int tile,
                                                             int staging, int max_words) {
     extern __shared__ uint32_t smem[];
-    const Lanes<G> L;
+    const BlockSmem B(smem, max_words);
     const int nframes = hdr->nframes;
     const int total = ray_start[nframes];
-    uint32_t* mask_words = smem + L.slot * max_words;
-    const BlockSmem B(smem, max_words, (static_cast<int>(blockDim.x) >> 5) * (32 / G), L.slot, G);
     Counts cnt;
     int f = 0;  // frame of the current ray (rays are taken in increasing order)
-    // Guided self-scheduling: a group claims up to `tile` adjacent rays, but
+    // Guided self-scheduling: a warp claims up to `tile` adjacent rays, but
     // never more than half its fair share of what is left, so the last rays
-    // go out one at a time and no group is left with a long private tail.
+    // go out one at a time and no warp is left with a long private tail.
     const int grab = tile;
-    const int groups = static_cast<int>(gridDim.x) * (static_cast<int>(blockDim.x) / G);
+    const int warps = static_cast<int>(gridDim.x) * B.slots;
     for (;;) {
         unsigned int t0 = 0, n = 1;
-        if (L.k == 0) {
+        if (B.k == 0) {
             const int seen = static_cast<int>(*reinterpret_cast<volatile unsigned int*>(&hdr->next_ray));
-            n = static_cast<unsigned int>(max(1, min(grab, (total - seen) / (2 * groups))));
+            n = static_cast<unsigned int>(max(1, min(grab, (total - seen) / (2 * warps))));
             t0 = atomicAdd(&hdr->next_ray, n);
         }
-        t0 = __shfl_sync(L.gmask, t0, lane_base(L.gmask));
-        n = __shfl_sync(L.gmask, n, lane_base(L.gmask));
+        t0 = __shfl_sync(kWarp, t0, 0);
+        n = __shfl_sync(kWarp, n, 0);
         if (static_cast<int>(t0) >= total) break;
         const int t1 = min(static_cast<int>(t0) + static_cast<int>(n), total);
         for (int r = static_cast<int>(t0); r < t1; r++) {
@@ -1364,29 +1337,29 @@ __global__ void __launch_bounds__(128, 4) raycast_batch_kernel(BatchHeader* hdr,
                 }
                 f = lo;
             }
-            cast_ray<G, false, kHits, kStage>(frames[f], r - ray_start[f], true, mask_words, B.recs, B.spans, B.list,
-                                              L.k, L.gmask, staging, cnt);
+            cast_ray<false, kHits, kStage>(frames[f], r - ray_start[f], true, B.mask, B.recs, B.spans, B.list, B.k,
+                                           staging, cnt);
         }
     }
 }
 
-template <int G, bool kCount, bool kHits, bool kStage>
+template <bool kCount, bool kHits, bool kStage>
 rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) {
     const int words = (p.S + 31) >> 5;
-    const int rays_per_block = threads / 32 * (32 / G);
+    const int rays_per_block = threads / kLanes;
     const size_t smem = raycast_smem_bytes(threads, rays_per_block, words);
     if (smem > 227 * 1024) {
         set_error("rle_render_rays: %d samples per ray exceed shared memory at this launch shape", p.S);
         return RLE_ERR_CAPACITY;
     }
-    cudaError_t e = cudaFuncSetAttribute(raycast_kernel<G, kCount, kHits, kStage>,
+    cudaError_t e = cudaFuncSetAttribute(raycast_kernel<kCount, kHits, kStage>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) {
         set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         return RLE_ERR_CUDA;
     }
     const int blocks = (p.rays + rays_per_block - 1) / rays_per_block;
-    raycast_kernel<G, kCount, kHits, kStage><<<blocks, threads, smem, stream>>>(p);
+    raycast_kernel<kCount, kHits, kStage><<<blocks, threads, smem, stream>>>(p);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("raycast launch: %s", cudaGetErrorString(e));
@@ -1395,40 +1368,38 @@ rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) 
     return RLE_OK;
 }
 
-template <int G, bool kStage>
+template <bool kStage>
 rle_status launch_output(const RayParams& p, int threads, cudaStream_t stream) {
-    return p.rayhit ? launch_variant<G, false, true, kStage>(p, threads, stream)
-                    : launch_variant<G, false, false, kStage>(p, threads, stream);
+    return p.rayhit ? launch_variant<false, true, kStage>(p, threads, stream)
+                    : launch_variant<false, false, kStage>(p, threads, stream);
 }
 
-template <int G>
 rle_status launch_shape(const RayParams& p, int threads, cudaStream_t stream) {
     if (p.counters) {  // the counts do not depend on the staging depth
-        return p.rayhit ? launch_variant<G, true, true, false>(p, threads, stream)
-                        : launch_variant<G, true, false, false>(p, threads, stream);
+        return p.rayhit ? launch_variant<true, true, false>(p, threads, stream)
+                        : launch_variant<true, false, false>(p, threads, stream);
     }
-    return p.staging >= 2 ? launch_output<G, true>(p, threads, stream) : launch_output<G, false>(p, threads, stream);
+    return p.staging >= 2 ? launch_output<true>(p, threads, stream) : launch_output<false>(p, threads, stream);
 }
 
-template <int G>
 size_t batch_smem(int threads, int max_samples) {
-    return raycast_smem_bytes(threads, threads / 32 * (32 / G), (max_samples + 31) >> 5);
+    return raycast_smem_bytes(threads, threads / kLanes, (max_samples + 31) >> 5);
 }
 
-template <int G, bool kHits, bool kStage>
+template <bool kHits, bool kStage>
 rle_status batch_blocks(int threads, int max_samples, int* blocks) {
-    const size_t smem = batch_smem<G>(threads, max_samples);
+    const size_t smem = batch_smem(threads, max_samples);
     if (smem > 227 * 1024) {
         set_error("batch: %d samples per ray exceed shared memory at this launch shape", max_samples);
         return RLE_ERR_CAPACITY;
     }
-    cudaError_t e = cudaFuncSetAttribute(raycast_batch_kernel<G, kHits, kStage>,
+    cudaError_t e = cudaFuncSetAttribute(raycast_batch_kernel<kHits, kStage>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     int dev = 0, sms = 0, per_sm = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raycast_batch_kernel<G, kHits, kStage>,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raycast_batch_kernel<kHits, kStage>,
                                                           threads, smem);
     if (e != cudaSuccess) {
         set_error("batch launch set-up: %s", cudaGetErrorString(e));
@@ -1438,15 +1409,15 @@ rle_status batch_blocks(int threads, int max_samples, int* blocks) {
     return RLE_OK;
 }
 
-template <int G, bool kHits, bool kStage>
+template <bool kHits, bool kStage>
 rle_status batch_launch(const BatchRaycast& b, cudaStream_t stream) {
-    const size_t smem = batch_smem<G>(b.threads, b.max_samples);
+    const size_t smem = batch_smem(b.threads, b.max_samples);
     int blocks = b.blocks;
     if (blocks <= 0) {
-        const rle_status st = batch_blocks<G, kHits, kStage>(b.threads, b.max_samples, &blocks);
+        const rle_status st = batch_blocks<kHits, kStage>(b.threads, b.max_samples, &blocks);
         if (st != RLE_OK) return st;
     }
-    raycast_batch_kernel<G, kHits, kStage><<<blocks, b.threads, smem, stream>>>(
+    raycast_batch_kernel<kHits, kStage><<<blocks, b.threads, smem, stream>>>(
         b.header, b.ray_start, b.frames, b.tile, b.staging, (b.max_samples + 31) >> 5);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1456,34 +1427,24 @@ rle_status batch_launch(const BatchRaycast& b, cudaStream_t stream) {
     return RLE_OK;
 }
 
-template <int G>
 rle_status batch_blocks_for(int threads, int max_samples, bool hits, bool stage, int* blocks) {
     if (stage)
-        return hits ? batch_blocks<G, true, true>(threads, max_samples, blocks)
-                    : batch_blocks<G, false, true>(threads, max_samples, blocks);
-    return hits ? batch_blocks<G, true, false>(threads, max_samples, blocks)
-                : batch_blocks<G, false, false>(threads, max_samples, blocks);
+        return hits ? batch_blocks<true, true>(threads, max_samples, blocks)
+                    : batch_blocks<false, true>(threads, max_samples, blocks);
+    return hits ? batch_blocks<true, false>(threads, max_samples, blocks)
+                : batch_blocks<false, false>(threads, max_samples, blocks);
 }
 
-template <int G>
 rle_status batch_launch_for(const BatchRaycast& b, cudaStream_t s) {
     if (b.staging >= 2)
-        return b.hits ? batch_launch<G, true, true>(b, s) : batch_launch<G, false, true>(b, s);
-    return b.hits ? batch_launch<G, true, false>(b, s) : batch_launch<G, false, false>(b, s);
+        return b.hits ? batch_launch<true, true>(b, s) : batch_launch<false, true>(b, s);
+    return b.hits ? batch_launch<true, false>(b, s) : batch_launch<false, false>(b, s);
 }
 
 }  // namespace
 
-rle_status batch_grid_blocks(int lanes, int threads, int max_samples, bool hits, int staging, int* blocks) {
-    const bool stage = staging >= 2;
-    switch (lanes) {
-        case 8: return batch_blocks_for<8>(threads, max_samples, hits, stage, blocks);
-        case 16: return batch_blocks_for<16>(threads, max_samples, hits, stage, blocks);
-        case 32: return batch_blocks_for<32>(threads, max_samples, hits, stage, blocks);
-        default:
-            set_error("batch: lanes per ray must be 8, 16 or 32");
-            return RLE_ERR_INVALID_ARG;
-    }
+rle_status batch_grid_blocks(int threads, int max_samples, bool hits, int staging, int* blocks) {
+    return batch_blocks_for(threads, max_samples, hits, staging >= 2, blocks);
 }
 
 rle_status launch_raycast_batch(const BatchRaycast& b, void* stream) {
@@ -1491,15 +1452,7 @@ rle_status launch_raycast_batch(const BatchRaycast& b, void* stream) {
         set_error("batch: threads per block a multiple of 32 up to 128, tile >= 1, staging 1..3");
         return RLE_ERR_INVALID_ARG;
     }
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    switch (b.lanes) {
-        case 8: return batch_launch_for<8>(b, s);
-        case 16: return batch_launch_for<16>(b, s);
-        case 32: return batch_launch_for<32>(b, s);
-        default:
-            set_error("batch: lanes per ray must be 8, 16 or 32");
-            return RLE_ERR_INVALID_ARG;
-    }
+    return batch_launch_for(b, static_cast<cudaStream_t>(stream));
 }
 
 bool bounds_render(unsigned* out4, bool clear) {
@@ -1520,7 +1473,6 @@ bool bounds_render(unsigned* out4, bool clear) {
 rle_status launch_raycast(const RayParams& p, void* stream) {
     if (p.rays <= 0) return RLE_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int lanes = p.lanes_per_ray > 0 ? p.lanes_per_ray : 32;
     const int threads = p.threads_per_block > 0 ? p.threads_per_block : 128;
     if (threads % 32 != 0 || threads > 128) {
         set_error("raycast: threads per block must be a multiple of 32, at most 128");
@@ -1530,14 +1482,7 @@ rle_status launch_raycast(const RayParams& p, void* stream) {
         set_error("raycast: staging depth 1..3 (0 = default)");
         return RLE_ERR_INVALID_ARG;
     }
-    switch (lanes) {
-        case 8: return launch_shape<8>(p, threads, s);
-        case 16: return launch_shape<16>(p, threads, s);
-        case 32: return launch_shape<32>(p, threads, s);
-        default:
-            set_error("raycast: lanes per ray must be 8, 16 or 32");
-            return RLE_ERR_INVALID_ARG;
-    }
+    return launch_shape(p, threads, s);
 }
 
 }  // namespace rle

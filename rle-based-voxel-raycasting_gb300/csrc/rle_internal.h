@@ -104,11 +104,7 @@ struct RayParams {
     rle_hit* rayhit;
     rle_counters* counters;
     rle_ray_time* ray_time;       // per-ray start/end times (single-frame kernel), or null
-    // launch shape (0 = default): lanes cooperating on one ray, DDA steps
-    // each lane claims per chunk, block size
-    int lanes_per_ray;
-    int cells_per_lane;
-    int threads_per_block;
+    int threads_per_block;        // block size (0 = default)
     int staging;                  // staging depth of the column data (1..3; 0 = default)
 };
 
@@ -149,9 +145,8 @@ struct BatchRaycast {
     BatchHeader* header;       // device
     const int* ray_start;      // device array [nframes + 1], prefix of rays
     const RayParams* frames;   // device array [nframes]
-    int tile;                  // most adjacent rays a lane group claims at once
+    int tile;                  // most adjacent rays a warp claims at once
     int staging;               // staging depth of the column data (1..3)
-    int lanes;                 // lanes per ray: 8, 16, 32
     int threads;               // block size
     int max_samples;           // largest S of the frames the launch may see
     int blocks;                // grid size (0: fill the GPU)
@@ -175,7 +170,7 @@ rle_status batch_render_scenes(rle_batch* b, const rle_scene* const* scenes, con
                                void* stream, cudaEvent_t* frame_done = nullptr);
 size_t batch_capacity_words(const rle_batch* b);
 int batch_max_frames(const rle_batch* b);
-rle_status batch_grid_blocks(int lanes, int threads, int max_samples, bool hits, int staging, int* blocks);
+rle_status batch_grid_blocks(int threads, int max_samples, bool hits, int staging, int* blocks);
 
 // Bounds-check words of the device code (zeros when none fired); false in
 // builds without RLE_BOUNDS_CHECK.  read: flags, first index hit; clear

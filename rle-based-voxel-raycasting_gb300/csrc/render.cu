@@ -274,14 +274,14 @@ __device__ __forceinline__ bool setup_ray(const RayParams& P, int x, Ray& R, Dda
     return true;
 }
 
-// One DDA cell: the distances along the ray where it begins and ends, its
-// column and the column's table entry.
+// One DDA cell: the distance along the ray where it begins (it ends where the
+// next lane's begins), its column, x | z << 16 (for hit records), and the
+// column's table entry (zero past the ray's end).
 struct Cell {
-    float near, far;
+    float near;
     uint32_t ex, ey;
     int mip;
-    int vx, vz;
-    bool valid;
+    uint32_t vxz;
 };
 
 // A cell's projection: depth and screen numerator of its near edge at column
@@ -291,9 +291,9 @@ struct Edge {
 };
 
 // Candidate runs a lane records per cell for the merge (shared memory, one
-// uint4 per run).  Six: since the scan drops runs whose samples are all
-// taken, cells rarely have more candidates.
-constexpr int kRecs = 6;
+// uint4 per run).  Seven is what three bits count; a cell with more is walked,
+// 20 times the cost of a record (six: batches of 64 mixed frames 1.5% slower).
+constexpr int kRecs = 7;
 
 // A lane's last coloured sample, stored one pass late: the colour gather
 // (a dependent load) then overlaps the following work instead of stalling
@@ -345,7 +345,7 @@ __device__ __forceinline__ Span span_setup(float res_y2, const Ray& R, float pz,
 template <bool kCount>
 __device__ __forceinline__ void draw_span(const Mask& mask, int k, uint32_t* row, float* drow,
                                           rle_hit* hrow, const uint16_t* colours, uint64_t colour_room, int S, int y,
-                                          int scr_y2, const Span& sp, int mip, int vx, int vz, Pending& pend,
+                                          int scr_y2, const Span& sp, int mip, uint32_t vxz, Pending& pend,
                                           Counts& cnt) {
     const float u2dz = sp.u2dz, onedz2 = sp.onedz2;
     if constexpr (kCount) cnt.spans++;
@@ -383,8 +383,8 @@ __device__ __forceinline__ void draw_span(const Mask& mask, int k, uint32_t* row
             drow[yy] = depth;
             if (hrow) {
                 rle_hit h;
-                h.x = static_cast<uint16_t>(vx);
-                h.z = static_cast<uint16_t>(vz);
+                h.x = static_cast<uint16_t>(vxz & 0xffffu);
+                h.z = static_cast<uint16_t>(vxz >> 16);
                 h.y = static_cast<uint16_t>((sp.sg0 >> mip) + static_cast<int>(u - static_cast<uint32_t>(sp.texture)));
                 h.mip = static_cast<uint8_t>(mip);
                 h.flags = 1;
@@ -460,7 +460,7 @@ __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, con
         const Span sp = span_setup(res_y2, R, e.pz, e.py, sgs, sgf, tex, texture);
         const uint64_t cofs = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(nruns);
         const uint64_t room = cofs <= P.slab_words[c.mip] ? P.slab_words[c.mip] - cofs : 0u;
-        draw_span<kCount>(mask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, c.vx, c.vz,
+        draw_span<kCount>(mask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, c.vxz,
                              pend, cnt);
     }
 }
@@ -491,20 +491,19 @@ __device__ __forceinline__ void lod_switch(Walk& w, int nummaps) {
 
 // Derives the column of one DDA step's cell and starts the fetch of its table
 // entry (the value is first used one chunk later in the pipeline).
-__device__ __forceinline__ void cell_fetch(const RayParams& P, const Ray& R, bool valid, float near, float far,
-                                           float pbx, float pby, int ib, int mip, Cell& c) {
+__device__ __forceinline__ void cell_fetch(const RayParams& P, const Ray& R, bool valid, float near, float pbx, float pby,
+                                           int ib, int mip, Cell& c) {
     const int voxel_x = static_cast<int>(P.posx + pbx) + (ib ? 0 : R.fix_x);
     const int voxel_z = static_cast<int>(P.posz + pby) + (ib ? R.fix_z : 0);
+    const uint32_t vx = static_cast<uint32_t>(voxel_x & (P.gridx0 - 1)) >> mip;
+    const uint32_t vz = static_cast<uint32_t>(voxel_z & (P.gridz0 - 1)) >> mip;
     c.near = near;
-    c.far = far;
     c.mip = mip;
-    c.vx = (voxel_x & (P.gridx0 - 1)) >> mip;
-    c.vz = (voxel_z & (P.gridz0 - 1)) >> mip;
+    c.vxz = vx | (vz << 16);
     c.ex = 0;
     c.ey = 0;
-    c.valid = valid;
     if (valid) {
-        const uint32_t ti = static_cast<uint32_t>(c.vx) + (static_cast<uint32_t>(c.vz) << (P.log2x0 - mip));
+        const uint32_t ti = vx + (vz << (P.log2x0 - mip));
         const uint2 e =
             in_bounds(ti < P.table_cols[mip], kBoundsTable, ti) ? __ldg(&P.table[mip][ti]) : make_uint2(0u, 0u);
         c.ex = e.x;
@@ -764,13 +763,11 @@ __device__ __forceinline__ uint32_t from_place(int n) {
 // The cell of lane `from`, and its projection, in every lane.
 __device__ __forceinline__ Cell cell_of(const Cell& c, int from) {
     Cell r;
-    r.near = r.far = 0.0f;  // in the projection
+    r.near = 0.0f;  // in the projection
     r.ex = __shfl_sync(kWarp, c.ex, from);
     r.ey = __shfl_sync(kWarp, c.ey, from);
     r.mip = __shfl_sync(kWarp, c.mip, from);
-    r.vx = __shfl_sync(kWarp, c.vx, from);
-    r.vz = __shfl_sync(kWarp, c.vz, from);
-    r.valid = true;
+    r.vxz = __shfl_sync(kWarp, c.vxz, from);
     return r;
 }
 __device__ __forceinline__ Edge edge_of(const Edge& e, int from) {
@@ -828,7 +825,7 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
         const int mip = __shfl_sync(kWarp, c.mip, src);
         const uint32_t cofs = __shfl_sync(kWarp, c.ex + 2u + (c.ey & 0xffffu), src);
         uint32_t vxz = 0;
-        if (hrow) vxz = __shfl_sync(kWarp, static_cast<uint32_t>(c.vx) | (static_cast<uint32_t>(c.vz) << 16), src);
+        if (hrow) vxz = __shfl_sync(kWarp, c.vxz, src);
         unsigned walks = __ballot_sync(kWarp, walk);
         int start = 0;
         for (;;) {
@@ -843,17 +840,29 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
                     const uint32_t taken = mask.w[w >> 5];
                     if (taken == 0xffffffffu) continue;
                     const uint32_t bits = in ? from_place(lo - w) & ~from_place(hi - w) : 0u;
-                    uint32_t before = __shfl_up_sync(kWarp, bits, 1);
-                    if (k == 0) before = 0u;
+                    // the first span here, and whether it alone counts: it covers the
+                    // word, or no other span reaches it (the inside of long spans)
+                    const unsigned reach = __ballot_sync(kWarp, bits != 0u);
+                    const unsigned whole = __ballot_sync(kWarp, bits == 0xffffffffu);
+                    uint32_t own = bits & ~taken, all;
+                    if ((reach & (reach - 1u)) == 0u || (whole & reach & (0u - reach)) != 0u) {
+                        const int f = __ffs(reach) - 1;
+                        all = __shfl_sync(kWarp, bits, max(f, 0));
+                        if (k != f) own = 0u;
+                    } else {
+                        uint32_t before = __shfl_up_sync(kWarp, bits, 1);
+                        if (k == 0) before = 0u;
 #pragma unroll
-                    for (int o = 1; o < kLanes; o <<= 1) {
-                        const uint32_t v = __shfl_up_sync(kWarp, before, o);
-                        if (k >= o) before |= v;
+                        for (int o = 1; o < kLanes; o <<= 1) {
+                            const uint32_t v = __shfl_up_sync(kWarp, before, o);
+                            if (k >= o) before |= v;
+                        }
+                        own &= ~before;
+                        all = __reduce_or_sync(kWarp, bits);
                     }
-                    const uint32_t own = bits & ~before & ~taken;
                     const unsigned claims = __ballot_sync(kWarp, own != 0u);
                     if (!claims) continue;
-                    mask.w[w >> 5] = taken | __reduce_or_sync(kWarp, bits);  // by every lane, the same word
+                    mask.w[w >> 5] = taken | all;  // by every lane, the same word
                     const int m = __popc(claims);
                     if (q.n + m > kLanes) flush_spans(P, R, q, k, row, drow, hrow, pend);
                     if (own) {
@@ -906,7 +915,7 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
 // (cell_alive) and the word-wise merge, per frame: 1920x1080 438 -> 310 us,
 // 1366x768 with hits 278 -> 225 us, 640x480 152 -> 130 us, 320x240 87 -> 82 us.
 struct ChunkStep {
-    float near, far, pbx, pby;
+    float near, pbx, pby;
     int ib, mip;
 };
 
@@ -926,36 +935,47 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, Chu
     float c_dd = 0, c_px = 0, c_py = 0;
     int c_ix = 0, smip = W.mip;
     int nvalid = kLanes;
-    bool done = false;
+    int pos = 0;  // steps taken
+    int jumps = W.z == 0.0f ? 0 : 3;
     if (W.cached && W.room >= kLanes) {
         const DdaJump j = dda_jump(W.d, W.c, static_cast<float>(k));
         const unsigned bad = __ballot_sync(kWarp, !j.ok);
         const unsigned kept = __ballot_sync(kWarp, j.kept);
-        const int src = kLanes - 1;
-        const float dd0 = __shfl_sync(kWarp, j.dd0, src), dd1 = __shfl_sync(kWarp, j.dd1, src);
-        const float i0x = __shfl_sync(kWarp, j.i0x, src), i0y = __shfl_sync(kWarp, j.i0y, src);
-        const float i1x = __shfl_sync(kWarp, j.i1x, src), i1y = __shfl_sync(kWarp, j.i1y, src);
+        float dd0 = __shfl_sync(kWarp, j.dd0, kLanes - 1), dd1 = __shfl_sync(kWarp, j.dd1, kLanes - 1);
+        float i0x = __shfl_sync(kWarp, j.i0x, kLanes - 1), i0y = __shfl_sync(kWarp, j.i0y, kLanes - 1);
+        float i1x = __shfl_sync(kWarp, j.i1x, kLanes - 1), i1y = __shfl_sync(kWarp, j.i1y, kLanes - 1);
         c_dd = j.dd;
         c_px = j.px;
         c_py = j.py;
         c_ix = j.axis1 ? 1 : 0;
-        done = bad == 0u;
-        if (done) {
+        pos = kLanes;
+        W.cached = kept >> 31;
+        if (bad) {  // up to the lane that is the first out of place; its event is right
+            pos = __ffs(bad);
+            const int src = max(pos - 2, 0);
+            dd0 = __shfl_sync(kWarp, j.dd0, src);
+            dd1 = __shfl_sync(kWarp, j.dd1, src);
+            i0x = __shfl_sync(kWarp, j.i0x, src);
+            i0y = __shfl_sync(kWarp, j.i0y, src);
+            i1x = __shfl_sync(kWarp, j.i1x, src);
+            i1y = __shfl_sync(kWarp, j.i1y, src);
+            W.cached = false;
+        }
+        if (pos > 1) {
             W.d.dd0 = dd0;
             W.d.dd1 = dd1;
             W.d.i0x = i0x;
             W.d.i0y = i0y;
             W.d.i1x = i1x;
             W.d.i1y = i1y;
-            W.cached = (kept >> src) & 1u;
-            W.z += W.dz * static_cast<float>(kLanes);
-            W.room -= kLanes;
         }
+        if (bad) dda_step(W.d);
+        W.z += W.dz * static_cast<float>(pos);
+        W.room -= pos;
+        jumps = 2;
     }
-    if (!done) {
+    if (pos < kLanes) {
         const float zfar = static_cast<float>(P.z_far);
-        int jumps = W.z == 0.0f ? 0 : 3;
-        int pos = 0;  // steps taken
 #pragma unroll 1
         while (pos < kLanes) {
             const int lim = min(kLanes, pos + W.room);
@@ -1044,7 +1064,6 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, Chu
     st.pbx = __shfl_sync(kWarp, last ? start_px : c_px, prev);
     st.pby = __shfl_sync(kWarp, last ? start_py : c_py, prev);
     st.ib = __shfl_sync(kWarp, last ? start_ix : c_ix, prev);
-    st.far = c_dd;
     st.mip = smip;
     return nvalid;
 }
@@ -1068,7 +1087,6 @@ __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, Chu
 struct Horizon {
     float a, b, eb;  // bound of f: a*t + b*h + eb*|h|
     float scene;     // b*h + eb*|h| of the scene's topmost voxel, or +inf
-    int ymin;
 };
 
 __device__ __forceinline__ Horizon horizon_bound(const RayParams& P, const Ray& R, int ymin) {
@@ -1086,15 +1104,14 @@ __device__ __forceinline__ Horizon horizon_bound(const RayParams& P, const Ray& 
     z.b = K * d + py_h;
     z.eb = z.b + eps * mb <= 0.0f ? eps * mb : INFINITY;  // inf: the bound drops nothing
     z.scene = z.a <= 0.0f ? z.b * h0 + z.eb * fabsf(h0) : INFINITY;
-    z.ymin = ymin;
     return z;
 }
 
 // Whether the cell may draw: it has runs and the topmost is not below the
 // horizon for good.
-__device__ __forceinline__ bool cell_alive(const RayParams& P, const Horizon& z, const Cell& c) {
+__device__ __forceinline__ bool cell_alive(const RayParams& P, const Horizon& z, const Cell& c, float far) {
     const float h = P.posy + static_cast<float>(static_cast<int>((c.ey >> 16) & 1023u) << c.mip);
-    const float bound = __fmaf_rn(z.a, z.a < 0.0f ? c.near : c.far, __fmaf_rn(z.b, h, z.eb * fabsf(h)));
+    const float bound = __fmaf_rn(z.a, z.a < 0.0f ? c.near : far, __fmaf_rn(z.b, h, z.eb * fabsf(h)));
     return (c.ey & 0xffffu) != 0u && !(bound < 0.0f);
 }
 
@@ -1155,7 +1172,7 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
         ChunkStep st;
         int nvalid = dda_chunk(P, W, k, st);
         Cell c;
-        cell_fetch(P, R, k < nvalid, st.near, st.far, st.pbx, st.pby, st.ib, st.mip, c);
+        cell_fetch(P, R, k < nvalid, st.near, st.pbx, st.pby, st.ib, st.mip, c);
         Horizon hz = horizon_bound(P, R, ymin);
         for (;;) {
             if (nvalid == 0) break;
@@ -1164,17 +1181,21 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             // issued now; their loads complete while this chunk is merged ----
             int nvalid_next = 0;
             Cell c_next;
+            c_next.near = 0.0f;
             if (!ended) {
                 ChunkStep st_next;
                 nvalid_next = dda_chunk(P, W, k, st_next);
-                cell_fetch(P, R, k < nvalid_next, st_next.near, st_next.far, st_next.pbx, st_next.pby, st_next.ib,
+                cell_fetch(P, R, k < nvalid_next, st_next.near, st_next.pbx, st_next.pby, st_next.ib,
                            st_next.mip, c_next);
             }
 
+            // a cell ends where the next lane's begins
+            const float far = __shfl_sync(kWarp, k == 0 ? c_next.near : c.near, (k + 1) % kLanes);
+
             if constexpr (kCount) {
                 // with counters every valid cell goes through the exact walk
-                const Edge edge = cell_edge(P, R, c.near, c.far);
-                unsigned todo = __ballot_sync(kWarp, c.valid);
+                const Edge edge = cell_edge(P, R, c.near, far);
+                unsigned todo = __ballot_sync(kWarp, k < nvalid);
                 // the reference ends the ray when its horizon closes, checked
                 // at every step before the cell (:370)
                 for (; todo && ymin < ymax; todo &= todo - 1) {
@@ -1185,15 +1206,16 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
                 }
             } else {
                 // ---- 2. each lane: its cell, unless it lies below the horizon ----
-                const bool alive = cell_alive(P, hz, c);
+                const bool alive = cell_alive(P, hz, c, far);
                 if (__ballot_sync(kWarp, alive)) {
-                    const Edge edge = cell_edge(P, R, c.near, c.far);
+                    const Edge edge = cell_edge(P, R, c.near, far);
+                    const int before = ymin;
                     int nrec = 0;
                     if (alive) nrec = scan_runs(P, R, mask, ymin, ymax, c, edge, my_recs, blockDim.x);
                     // ---- 3. the recorded runs, in the order of the walk ----
                     merge_chunk(P, R, mask, k, row, drow, hrow, c, edge, nrec, warp_recs, blockDim.x, list,
                                    ymin, ymax, pend, q, cnt);
-                    if (ymin != hz.ymin) hz = horizon_bound(P, R, ymin);
+                    if (ymin != before) hz = horizon_bound(P, R, ymin);
                 }
             }
             if (ymin >= ymax || ended) break;
@@ -1202,14 +1224,14 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
             // reference walks on to z_far without drawing).  Exact counters
             // need the full walk, so they keep it.
             if (!kCount) {
-                const float t_end = __shfl_sync(kWarp, c.far, kLanes - 1);
+                const float t_end = __shfl_sync(kWarp, far, kLanes - 1);
                 if (__fmaf_rn(hz.a, t_end, hz.scene) < 0.0f) break;
             }
             // staging depth >= 2: the next chunk's table entries have arrived
             // under the merge; stage each cell's header line (second header
             // on; the first travels in the table entry) for its scan, which
             // follows the next DDA chunk
-            if (kStage && c_next.valid && (c_next.ey & 0xffffu) > 1u)
+            if (kStage && (c_next.ey & 0xffffu) > 1u)
                 stage_headers(P.slabs[c_next.mip] + 3 + c_next.ex, staging);
             c = c_next;
             nvalid = nvalid_next;

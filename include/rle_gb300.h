@@ -261,11 +261,9 @@ typedef struct rle_counters {
  *                      every frame and batch
  *   cells_per_lane     DDA steps each lane takes per chunk: 1 (reserved)
  *   threads_per_block  32, 64, 96 or 128; default 128
- *   staging            staging depth of the column data a ray reads: 1 the
- *                      column-table entries of the next chunk of cells load
- *                      while the current chunk is merged; 2 also each of
- *                      those cells' run-header line is staged in L2 before
- *                      its scan; 3 the same into L1; default 1 */
+ *   staging            1, 2 or 3; default 1.  Accepted, without effect on the
+ *                      launch: column data is loaded under the next chunk's
+ *                      DDA, and staging it earlier measured no gain */
 typedef struct rle_tuning {
     int lanes_per_ray;
     int cells_per_lane;
@@ -358,7 +356,7 @@ typedef struct rle_batch_tuning {
     int tile_rays;          /* tile width: most adjacent column rays a warp claims at
                                once, 1..256 (default 1; claims shrink as the queue drains) */
     int lanes_per_ray;      /* 8, 16 or 32, as rle_tuning.lanes_per_ray */
-    int staging;            /* staging depth of the column data, 1..3, as rle_tuning.staging */
+    int staging;            /* 1..3, as rle_tuning.staging */
     int threads_per_block;  /* 32, 64, 96 or 128 */
     int use_graph;          /* 1: capture once and replay (default); 0: plain launches */
     int per_frame;          /* 1 (default): one plain raycast + resolve launch pair per frame,
@@ -383,10 +381,9 @@ size_t rle_batch_words_needed(const rle_frame_request* frames, int n);
  * the batch's ray buffer and parameter block), whatever streams they use. */
 rle_status rle_batch_render(rle_batch* b, const rle_scene* scene, const rle_frame_request* frames, int n,
                             void* stream);
-/* Times every tile_rays x staging combination ({1,2,4,8,16,32,64} x {1,2,3}:
- * tile width, staging depth) and the per-frame launches (staging {1,2,3}) on
- * these frames (median of `repeats` runs each), keeps the fastest as the
- * batch's tuning and returns it. */
+/* Times every tile width ({1,2,4,8,16,32,64}) of the persistent pair and the
+ * per-frame launches on these frames (median of `repeats` runs each), keeps
+ * the fastest as the batch's tuning and returns it. */
 rle_status rle_batch_autotune(rle_batch* b, const rle_scene* scene, const rle_frame_request* frames, int n,
                               int repeats, rle_batch_tuning* best, float* best_ms);
 

@@ -122,7 +122,7 @@ void release(rle_batch* b) {
 
 rle_status prepare_grid(rle_batch* b) {
     rle_status st = rle::batch_grid_blocks(b->tuning.threads_per_block, b->max_samples,
-                                           b->with_hits, b->tuning.staging, &b->raycast_blocks);
+                                           b->with_hits, &b->raycast_blocks);
     if (st != RLE_OK) return st;
     int sms = 0;
     const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
@@ -210,7 +210,6 @@ rle_status enqueue(rle_batch* b, int parity, cudaStream_t s) {
     rc.ray_start = reinterpret_cast<const int*>(b->d_params + L.ray_start);
     rc.frames = reinterpret_cast<const rle::RayParams*>(b->d_params + L.ray_params);
     rc.tile = b->tuning.tile_rays;
-    rc.staging = b->tuning.staging;
     rc.threads = b->tuning.threads_per_block;
     rc.max_samples = b->max_samples;
     rc.blocks = b->raycast_blocks;
@@ -264,7 +263,6 @@ rle_status render_locked(rle_batch* b, const rle_scene* scene, const rle_scene* 
         if (e != cudaSuccess) return cuda_fail(e, "rle_batch_render: fork to the worker streams");
         for (int i = 0; i < n && st == RLE_OK; i++) {
             rp[i].threads_per_block = b->tuning.threads_per_block;
-            rp[i].staging = b->tuning.staging;
             st = rle::launch_raycast(rp[i], b->workers[i % k]);
             if (st == RLE_OK) st = rle::launch_resolve(sp[i], b->workers[i % k]);
             if (st == RLE_OK && frame_done && cudaEventRecord(frame_done[i], b->workers[i % k]) != cudaSuccess)
@@ -472,35 +470,32 @@ extern "C" rle_status rle_batch_autotune(rle_batch* b, const rle_scene* scene, c
     rle_batch_tuning win = start;
     float win_ms = 1e30f;
     rle_status st = RLE_OK;
-    // the persistent launch over tile x staging, then the per-frame launches (tile -1)
+    // the persistent launch over the tile widths, then the per-frame launches (tile -1)
     for (int tv : {1, 2, 4, 8, 16, 32, 64, -1}) {
-        for (int sv : {1, 2, 3}) {
-            rle_batch_tuning t = start;
-            t.per_frame = tv < 0 ? 1 : 0;
-            t.tile_rays = tv < 0 ? start.tile_rays : tv;
-            t.lanes_per_ray = 32;
-            t.staging = sv;
-            if ((st = rle_batch_set_tuning(b, &t)) != RLE_OK) break;
-            if ((st = rle_batch_render(b, scene, frames, n, s)) != RLE_OK) break;  // warm-up / capture
-            std::vector<float> ms;
-            for (int r = 0; r < repeats && st == RLE_OK; r++) {
-                cudaEventRecord(e0, s);
-                st = rle_batch_render(b, scene, frames, n, s);
-                cudaEventRecord(e1, s);
-                cudaEventSynchronize(e1);
-                float v = 0;
-                cudaEventElapsedTime(&v, e0, e1);
-                ms.push_back(v);
-            }
-            if (st != RLE_OK) break;
-            std::nth_element(ms.begin(), ms.begin() + ms.size() / 2, ms.end());
-            const float med = ms[ms.size() / 2];
-            if (med < win_ms) {
-                win_ms = med;
-                win = t;
-            }
+        rle_batch_tuning t = start;
+        t.per_frame = tv < 0 ? 1 : 0;
+        t.tile_rays = tv < 0 ? start.tile_rays : tv;
+        t.lanes_per_ray = 32;
+        t.staging = 1;
+        if ((st = rle_batch_set_tuning(b, &t)) != RLE_OK) break;
+        if ((st = rle_batch_render(b, scene, frames, n, s)) != RLE_OK) break;  // warm-up / capture
+        std::vector<float> ms;
+        for (int r = 0; r < repeats && st == RLE_OK; r++) {
+            cudaEventRecord(e0, s);
+            st = rle_batch_render(b, scene, frames, n, s);
+            cudaEventRecord(e1, s);
+            cudaEventSynchronize(e1);
+            float v = 0;
+            cudaEventElapsedTime(&v, e0, e1);
+            ms.push_back(v);
         }
         if (st != RLE_OK) break;
+        std::nth_element(ms.begin(), ms.begin() + ms.size() / 2, ms.end());
+        const float med = ms[ms.size() / 2];
+        if (med < win_ms) {
+            win_ms = med;
+            win = t;
+        }
     }
     cudaStreamSynchronize(s);
     cudaEventDestroy(e0);

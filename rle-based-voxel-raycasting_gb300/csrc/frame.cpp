@@ -181,7 +181,6 @@ extern "C" rle_status rle_render_rays(const rle_scene* scene, const rle_raymap* 
     p.rayhit = d_rayhit;
     p.counters = d_counters;
     p.threads_per_block = g_threads_per_block;
-    p.staging = g_staging;
     rle::DeviceGuard g(scene->device);
     if (!g.ok) {
         rle::set_error("rle_render_rays: cannot select device %d", scene->device);
@@ -203,7 +202,6 @@ extern "C" rle_status rle_render_rays_timed(const rle_scene* scene, const rle_ra
     p.raydepth = d_raydepth;
     p.ray_time = d_times;
     p.threads_per_block = g_threads_per_block;
-    p.staging = g_staging;
     rle::DeviceGuard g(scene->device);
     if (!g.ok) {
         rle::set_error("rle_render_rays_timed: cannot select device %d", scene->device);

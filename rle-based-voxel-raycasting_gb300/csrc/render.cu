@@ -108,15 +108,6 @@ __device__ __forceinline__ uint32_t sm_id() {
     return s;
 }
 
-// Run-header staging (staging depth 2 or 3; the variants built with kStage):
-// 2 stages a cell's header line in L2, 3 in L1, ahead of the scan that reads
-// it.  Depth 1 variants carry none of this code: a runtime test in the chunk
-// loop measured 1% slower single frames and 4% slower batches at depth 1.
-__device__ __forceinline__ void stage_headers(const uint16_t* h, int staging) {
-    if (staging == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(h));
-    else if (staging >= 3) asm volatile("prefetch.global.L1 [%0];" ::"l"(h));
-}
-
 // One warp owns one ray.  (Two or four rays per warp share its instructions
 // only while they take the same branches; the chunk that draws, the jump that
 // ends early and the ray that ends are branches.  Measured on batches, 8 / 16 /
@@ -275,14 +266,21 @@ __device__ __forceinline__ bool setup_ray(const RayParams& P, int x, Ray& R, Dda
 }
 
 // One DDA cell: the distance along the ray where it begins (it ends where the
-// next lane's begins), its column, x | z << 16 (for hit records), and the
-// column's table entry (zero past the ray's end).
+// next lane's begins), its level (-1 past the ray's end), its column's index
+// there, and the column's table entry.
 struct Cell {
     float near;
-    uint32_t ex, ey;
     int mip;
-    uint32_t vxz;
+    uint32_t column;
+    uint32_t ex, ey;
 };
+
+// Its column's coordinates, x | z << 16, as hit records have them.
+__device__ __forceinline__ uint32_t cell_xz(const RayParams& P, const Cell& c) {
+    const int shift = P.log2x0 - c.mip;
+    return (c.column & ((1u << shift) - 1u)) | ((c.column >> shift) << 16);
+}
+
 
 // A cell's projection: depth and screen numerator of its near edge at column
 // index 0, and what its far edge adds.
@@ -290,8 +288,8 @@ struct Edge {
     float pz, py, czz, cyy;
 };
 
-// Candidate runs a lane records per cell for the merge (shared memory, one
-// uint4 per run).  Seven is what three bits count; a cell with more is walked,
+// Candidate runs a lane records per cell for the merge (shared memory, three
+// words per run).  Seven is what three bits count; a cell with more is walked,
 // 20 times the cost of a record (six: batches of 64 mixed frames 1.5% slower).
 constexpr int kRecs = 7;
 
@@ -315,13 +313,13 @@ struct Span {
     int texture, sg0;
 };
 
-__device__ __forceinline__ Span span_setup(float res_y2, const Ray& R, float pz, float py, float sgs, float sgf,
+__device__ __forceinline__ Span span_setup(float res_y2, float z_add, float y_add, float pz, float py, float sgs, float sgf,
                                            float tex, int texture) {
     Span sp;
-    const float pz1r = pz + R.pos3d_z_add * sgs;
-    const float py1r = py + R.pos3d_y_add * sgs;
-    const float pz2r = pz + R.pos3d_z_add * sgf;
-    const float py2r = py + R.pos3d_y_add * sgf;
+    const float pz1r = pz + z_add * sgs;
+    const float py1r = py + y_add * sgs;
+    const float pz2r = pz + z_add * sgf;
+    const float py2r = py + y_add * sgf;
     const float scr_y2r = res_y2 + py1r / pz1r;
     const float scr_y1r = res_y2 + py2r / pz2r;
     const float u1z = tex / pz2r;
@@ -403,8 +401,9 @@ __device__ __forceinline__ void draw_span(const Mask& mask, int k, uint32_t* row
 template <bool kCount>
 __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, const Mask& mask, int k,
                                            uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, const Edge& e, int& ymin,
-                                           int& ymax, Pending& pend, Counts& cnt) {
+                                           int& ymax, Counts& cnt) {
     const float res_y2 = static_cast<float>(P.S / 2);
+    Pending pend;
     // clip top (:467)
     if (e.pz * res_y2 + e.py <= e.pz * static_cast<float>(ymin)) return;
     if constexpr (kCount) cnt.fetched++;
@@ -457,12 +456,13 @@ __device__ __forceinline__ void merge_cell(const RayParams& P, const Ray& R, con
         }
         const int y = mask.first_clear(scr_y1, scr_y2);
         if (y >= scr_y2) continue;
-        const Span sp = span_setup(res_y2, R, e.pz, e.py, sgs, sgf, tex, texture);
+        const Span sp = span_setup(res_y2, R.pos3d_z_add, R.pos3d_y_add, e.pz, e.py, sgs, sgf, tex, texture);
         const uint64_t cofs = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(nruns);
         const uint64_t room = cofs <= P.slab_words[c.mip] ? P.slab_words[c.mip] - cofs : 0u;
-        draw_span<kCount>(mask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, c.vxz,
+        draw_span<kCount>(mask, k, row, drow, hrow, colours, room, P.S, y, scr_y2, sp, c.mip, cell_xz(P, c),
                              pend, cnt);
     }
+    pend.flush();
 }
 
 
@@ -489,26 +489,33 @@ __device__ __forceinline__ void lod_switch(Walk& w, int nummaps) {
     }
 }
 
-// Derives the column of one DDA step's cell and starts the fetch of its table
-// entry (the value is first used one chunk later in the pipeline).
-__device__ __forceinline__ void cell_fetch(const RayParams& P, const Ray& R, bool valid, float near, float pbx, float pby,
-                                           int ib, int mip, Cell& c) {
-    const int voxel_x = static_cast<int>(P.posx + pbx) + (ib ? 0 : R.fix_x);
-    const int voxel_z = static_cast<int>(P.posz + pby) + (ib ? R.fix_z : 0);
-    const uint32_t vx = static_cast<uint32_t>(voxel_x & (P.gridx0 - 1)) >> mip;
-    const uint32_t vz = static_cast<uint32_t>(voxel_z & (P.gridz0 - 1)) >> mip;
-    c.near = near;
-    c.mip = mip;
-    c.vxz = vx | (vz << 16);
-    c.ex = 0;
-    c.ey = 0;
-    if (valid) {
-        const uint32_t ti = vx + (vz << (P.log2x0 - mip));
-        const uint2 e =
-            in_bounds(ti < P.table_cols[mip], kBoundsTable, ti) ? __ldg(&P.table[mip][ti]) : make_uint2(0u, 0u);
-        c.ex = e.x;
-        c.ey = e.y;
-    }
+// What a DDA step gives for its cell.
+struct ChunkStep {
+    float near, pbx, pby;
+    int ib, mip;
+};
+
+// The cell of one DDA step.  Its table entry is loaded at the top of its own
+// turn of the chunk loop, under the next chunk's DDA: loaded a turn earlier, its
+// registers are waited for where the loop hands them on, which was a sixth of
+// a slow ray's time (1920x1080 frames 313 -> 279 us; staged in L1 or L2 a turn
+// earlier as well: no gain, nor through asynchronous copies to shared memory).
+__device__ __forceinline__ Cell cell_of_step(const RayParams& P, const Ray& R, bool valid, const ChunkStep& st) {
+    const int voxel_x = static_cast<int>(P.posx + st.pbx) + (st.ib ? 0 : R.fix_x);
+    const int voxel_z = static_cast<int>(P.posz + st.pby) + (st.ib ? R.fix_z : 0);
+    const uint32_t vx = static_cast<uint32_t>(voxel_x & (P.gridx0 - 1)) >> st.mip;
+    const uint32_t vz = static_cast<uint32_t>(voxel_z & (P.gridz0 - 1)) >> st.mip;
+    Cell c;
+    c.near = st.near;
+    c.mip = valid ? st.mip : -1;
+    c.column = vx + (vz << (P.log2x0 - st.mip));
+    return c;
+}
+
+__device__ __forceinline__ uint2 cell_entry(const RayParams& P, const Cell& c) {
+    return c.mip >= 0 && in_bounds(c.column < P.table_cols[c.mip], kBoundsTable, c.column)
+               ? __ldg(&P.table[c.mip][c.column])
+               : make_uint2(0u, 0u);
 }
 
 __device__ __forceinline__ Edge cell_edge(const RayParams& P, const Ray& R, float near, float far) {
@@ -532,7 +539,8 @@ __device__ __forceinline__ Edge cell_edge(const RayParams& P, const Ray& R, floa
 // Pre-culls a cell against the horizon at the start of its chunk and scans
 // its runs.  Returns the number of runs recorded in `rec` (one slot every
 // `stride` entries) that the exact walk could still draw, or -1 if the cell
-// has to be walked run by run at its turn.
+// has to be walked run by run at its turn.  Run headers are loaded two runs
+// ahead (the first travels in the table entry).
 //
 // A run is recorded unless, at the chunk's horizon, the walk would skip it for
 // good (`pz1 <= 0`, `pz2 <= 0`, `scr_y1 >= ymax`) or none of its samples in the
@@ -553,16 +561,14 @@ __device__ __forceinline__ Edge cell_edge(const RayParams& P, const Ray& R, floa
 //    the last horizon at which a recorded run still has a sample above it
 //    (for pz >= 0 it gets truer as ymin grows, for pz < 0 less true).
 __device__ __forceinline__ int scan_runs(const RayParams& P, const Ray& R, const Mask& mask, int ymin, int ymax,
-                                         const Cell& c, const Edge& e, uint4* rec, int stride) {
+                                         const Cell& c, const Edge& e, uint32_t* rec, int stride) {
     const float res_y2 = static_cast<float>(P.S / 2);
     const float mountain = P.posy;
     const int mip = c.mip;
     // clip top at the current horizon
     if (e.pz >= 0.0f && e.pz * res_y2 + e.py <= e.pz * static_cast<float>(ymin)) return 0;
-    const uint16_t* hdr = P.slabs[mip] + 2 + c.ex;
     const int nruns = c.ey & 0xffffu;
-    // headers are loaded two runs ahead: the first arrives with the table
-    // entry, and each later one would cost its latency in turn
+    const uint16_t* hdr = P.slabs[mip] + 2 + c.ex;
     auto header = [&](int r) -> uint32_t {
         const uint64_t hi = static_cast<uint64_t>(c.ex) + 2u + static_cast<uint64_t>(r);
         return r < nruns && in_bounds(hi < P.slab_words[mip], kBoundsHeader, hi) ? __ldg(&hdr[r]) : 0u;
@@ -602,9 +608,9 @@ __device__ __forceinline__ int scan_runs(const RayParams& P, const Ray& R, const
         const int lo = mask.first_clear(max(scr_y1, ymin), hi);
         if (lo >= hi) continue;  // every sample it could colour is taken already
         if (n == kRecs || scr_y2 != low) return -1;
-        rec[n * stride] = make_uint4(static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16),
-                                     static_cast<uint32_t>(start),
-                                     static_cast<uint32_t>(texture) | (static_cast<uint32_t>(solid) << 16), 0u);
+        rec[(3 * n) * stride] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+        rec[(3 * n + 1) * stride] = static_cast<uint32_t>(start);
+        rec[(3 * n + 2) * stride] = static_cast<uint32_t>(texture) | (static_cast<uint32_t>(solid) << 16);
         top = max(top, hi);
         n++;
     }
@@ -650,13 +656,13 @@ __device__ __forceinline__ int nth_bit(uint32_t m, int r) {
     return at;
 }
 
-__device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, SpanQueue& q, int k,
-                                            uint32_t* row, float* drow, rle_hit* hrow, Pending& pend) {
-    if (q.n == 0) return;
+__device__ __forceinline__ void flush_spans(const RayParams& P, float z_add, float y_add, uint4* queue, int n, int k,
+                                            uint32_t* row, float* drow, rle_hit* hrow) {
+    Pending pend;
     uint4 e0 = make_uint4(0u, 0u, 0u, 0u), e1 = e0;
-    if (k < q.n) {
-        e0 = q.e[k];
-        e1 = q.e[kLanes + k];
+    if (k < n) {
+        e0 = queue[k];
+        e1 = queue[kLanes + k];
     }
     // samples per queued piece, inclusive prefix over the lanes
     const int cnt = __popc(e0.y);
@@ -666,15 +672,15 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
         const int v = __shfl_up_sync(kWarp, incl, o);
         if (k >= o) incl += v;
     }
-    const int total = __shfl_sync(kWarp, incl, q.n - 1);
+    const int total = __shfl_sync(kWarp, incl, n - 1);
     const int start = incl - cnt;
     // this lane's piece: the accumulators at its first sample and their step,
     // rounded (the sums are then one multiply-add away) or, where they leave
     // their binade within the piece, as it is
-    if (k < q.n) {
+    if (k < n) {
         const int sg = static_cast<int>(e1.z), texture = static_cast<int>(e0.w & 0xffffu);
         const int solid = static_cast<int>(e0.w >> 16), mip = static_cast<int>(e0.x >> 28);
-        const Span sp = span_setup(static_cast<float>(P.S / 2), R, __uint_as_float(e1.x), __uint_as_float(e1.y),
+        const Span sp = span_setup(static_cast<float>(P.S / 2), z_add, y_add, __uint_as_float(e1.x), __uint_as_float(e1.y),
                                    static_cast<float>(sg), static_cast<float>(sg + (solid << mip)),
                                    static_cast<float>(texture + solid), texture);
         const int y0 = static_cast<int>(e0.x & 0x3fffu), skip = static_cast<int>((e0.x >> 14) & 0x3fffu) - y0;
@@ -684,8 +690,8 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
         const int steps = 31 - __clz(static_cast<int>(e0.y));  // to the piece's last claimed sample
         float du, dz;
         const bool jump = steady_step(uz, sp.u2dz, steps, &du) & steady_step(onez, sp.onedz2, steps, &dz);
-        q.e[k].x = e0.x | (jump ? 0x80000000u : 0u);
-        q.e[kLanes + k] = make_uint4(bits_of(uz), bits_of(jump ? du : sp.u2dz), bits_of(onez),
+        queue[k].x = e0.x | (jump ? 0x80000000u : 0u);
+        queue[kLanes + k] = make_uint4(bits_of(uz), bits_of(jump ? du : sp.u2dz), bits_of(onez),
                                 bits_of(jump ? dz : sp.onedz2));
     }
     __syncwarp();
@@ -695,7 +701,7 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
         // numbers (every queued piece owns at least one sample); those that
         // start at or before b, plus those starting in (b, b + k], count
         // the pieces at or before t
-        const bool entry = k < q.n;
+        const bool entry = k < n;
         unsigned le = __ballot_sync(kWarp, entry && start <= b);
         const unsigned marks =
             __reduce_or_sync(kWarp, (entry && start > b && start < b + kLanes) ? (1u << (start - b)) : 0u);
@@ -708,7 +714,7 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
             sg = __shfl_sync(kWarp, e1.z, from);
         }
         if (t < total) {
-            const uint4 v0 = q.e[from], v1 = q.e[kLanes + from];
+            const uint4 v0 = queue[from], v1 = queue[kLanes + from];
             const uint32_t at = v0.x, cofs = v0.z, tc = v0.w;
             const int mip = static_cast<int>((at >> 28) & 7u);
             const int steps = nth_bit(v0.y, t - before);
@@ -748,8 +754,8 @@ __device__ __forceinline__ void flush_spans(const RayParams& P, const Ray& R, Sp
             }
         }
     }
+    pend.flush();
     __syncwarp();  // the entries are rewritten by the next spans
-    q.n = 0;
 }
 
 // ~0 << max(n, 0), 0 from n = 32 on: the samples at or past place n of a
@@ -767,7 +773,7 @@ __device__ __forceinline__ Cell cell_of(const Cell& c, int from) {
     r.ex = __shfl_sync(kWarp, c.ex, from);
     r.ey = __shfl_sync(kWarp, c.ey, from);
     r.mip = __shfl_sync(kWarp, c.mip, from);
-    r.vxz = __shfl_sync(kWarp, c.vxz, from);
+    r.column = __shfl_sync(kWarp, c.column, from);
     return r;
 }
 __device__ __forceinline__ Edge edge_of(const Edge& e, int from) {
@@ -797,8 +803,8 @@ __device__ __forceinline__ Edge edge_of(const Edge& e, int from) {
 // (4700 -> 3000 cycles per chunk that draws; 1920x1080 frames 350 -> 310 us).
 __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, const Mask& mask, int k,
                                             uint32_t* row, float* drow, rle_hit* hrow, const Cell& c, const Edge& edge,
-                                            int nrec, const uint4* warp_recs, int stride, uint32_t* list, int& ymin,
-                                            int& ymax, Pending& pend, SpanQueue& q, Counts& cnt) {
+                                            int nrec, const uint32_t* warp_recs, int stride, uint32_t* list, int& ymin,
+                                            int& ymax, SpanQueue& q, Counts& cnt) {
     // entries before this lane's cell, and in all: its records (at most kRecs,
     // three bits), or one for a cell to walk
     const int mine = nrec < 0 ? 1 : nrec;
@@ -818,14 +824,19 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
         const uint32_t entry = k < n ? list[k] : 0u;
         const int src = k < n ? static_cast<int>(entry & 31u) : 0;
         const bool walk = (entry & 0x100u) != 0u;
-        uint4 rec = make_uint4(0u, 0u, 0u, 0u);
-        if (k < n && !walk) rec = warp_recs[static_cast<int>((entry >> 5) & 7u) * stride + src];
-        const int lo = static_cast<int>(rec.x & 0xffffu), hi = static_cast<int>(rec.x >> 16);
+        uint32_t range = 0u, begin = 0u, colours = 0u;
+        if (k < n && !walk) {
+            const uint32_t* rec = warp_recs + 3 * static_cast<int>((entry >> 5) & 7u) * stride + src;
+            range = rec[0];
+            begin = rec[stride];
+            colours = rec[2 * stride];
+        }
+        const int lo = static_cast<int>(range & 0xffffu), hi = static_cast<int>(range >> 16);
         const float pz = __shfl_sync(kWarp, edge.pz, src), py = __shfl_sync(kWarp, edge.py, src);
         const int mip = __shfl_sync(kWarp, c.mip, src);
         const uint32_t cofs = __shfl_sync(kWarp, c.ex + 2u + (c.ey & 0xffffu), src);
         uint32_t vxz = 0;
-        if (hrow) vxz = __shfl_sync(kWarp, c.vxz, src);
+        if (hrow) vxz = __shfl_sync(kWarp, cell_xz(P, c), src);
         unsigned walks = __ballot_sync(kWarp, walk);
         int start = 0;
         for (;;) {
@@ -864,15 +875,18 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
                     if (!claims) continue;
                     mask.w[w >> 5] = taken | all;  // by every lane, the same word
                     const int m = __popc(claims);
-                    if (q.n + m > kLanes) flush_spans(P, R, q, k, row, drow, hrow, pend);
+                    if (q.n + m > kLanes) {
+                        flush_spans(P, R.pos3d_z_add, R.pos3d_y_add, q.e, q.n, k, row, drow, hrow);
+                        q.n = 0;
+                    }
                     if (own) {
                         const int skip = __ffs(own) - 1, p0 = w + skip;
                         if (y0 < 0) y0 = p0;
                         uint4* e = q.e + q.n + __popc(claims & ((1u << k) - 1u));
                         e[0] = make_uint4(static_cast<uint32_t>(y0) | (static_cast<uint32_t>(p0) << 14) |
                                               (static_cast<uint32_t>(mip) << 28),
-                                          own >> skip, cofs, rec.z);
-                        e[kLanes] = make_uint4(__float_as_uint(pz), __float_as_uint(py), rec.y, vxz);
+                                          own >> skip, cofs, colours);
+                        e[kLanes] = make_uint4(__float_as_uint(pz), __float_as_uint(py), begin, vxz);
                     }
                     q.n += m;
                     __syncwarp();
@@ -887,7 +901,7 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
             start = stop + 1;
             const int from = __shfl_sync(kWarp, src, stop);
             merge_cell<false>(P, R, mask, k, row, drow, hrow, cell_of(c, from),
-                                 edge_of(edge, from), ymin, ymax, pend, cnt);
+                                 edge_of(edge, from), ymin, ymax, cnt);
             if (start >= n || ymin >= ymax) break;
         }
         __syncwarp();  // the list and the records are rewritten
@@ -914,11 +928,6 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
 // with the horizon test that drops whole chunks before they are projected
 // (cell_alive) and the word-wise merge, per frame: 1920x1080 438 -> 310 us,
 // 1366x768 with hits 278 -> 225 us, 640x480 152 -> 130 us, 320x240 87 -> 82 us.
-struct ChunkStep {
-    float near, pbx, pby;
-    int ib, mip;
-};
-
 // Steps from here that can meet neither a LOD switch nor the end of the ray.
 // z, dz (a power of two) and the switch distances are whole numbers held in
 // floats, exactly below 2^24.
@@ -1118,16 +1127,15 @@ __device__ __forceinline__ bool cell_alive(const RayParams& P, const Horizon& z,
 // Casts ray x of frame P with one warp (lane k), using mask_words (S/32 words
 // of shared memory) as its bitmask, in chunks of 32 DDA steps, lane k taking
 // step k of each.
-template <bool kCount, bool kHits, bool kStage>
-__device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active, uint32_t* mask_words, uint4* recs,
-                                         uint4* spans, uint32_t* list, int k, int staging, Counts& cnt) {
+template <bool kCount, bool kHits>
+__device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active, uint32_t* mask_words, uint32_t* recs,
+                                         uint4* spans, uint32_t* list, int k, Counts& cnt) {
     const int S = P.S;
     const int words = (S + 31) >> 5;
     Mask mask{mask_words};
 
-    uint4* my_recs = recs + threadIdx.x;
-    const uint4* warp_recs = recs + (threadIdx.x & ~31u);
-    Pending pend;
+    uint32_t* my_recs = recs + threadIdx.x;
+    const uint32_t* warp_recs = recs + (threadIdx.x & ~31u);
     SpanQueue q{spans, 0};
     Ray R;
     Walk W;
@@ -1171,25 +1179,24 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
         W.room = W.z > W.zswitch ? 0 : steps_unchecked(P, W);
         ChunkStep st;
         int nvalid = dda_chunk(P, W, k, st);
-        Cell c;
-        cell_fetch(P, R, k < nvalid, st.near, st.pbx, st.pby, st.ib, st.mip, c);
+        Cell c = cell_of_step(P, R, k < nvalid, st);
         Horizon hz = horizon_bound(P, R, ymin);
         for (;;) {
             if (nvalid == 0) break;
             const bool ended = nvalid < kLanes;
-            // ---- 1. the next chunk's DDA steps and column-table fetches are
-            // issued now; their loads complete while this chunk is merged ----
+            // ---- 1. this chunk's table entries, and under their latency the
+            // next chunk's DDA steps ----
+            const uint2 entry = cell_entry(P, c);
             int nvalid_next = 0;
             Cell c_next;
             c_next.near = 0.0f;
             if (!ended) {
-                ChunkStep st_next;
-                nvalid_next = dda_chunk(P, W, k, st_next);
-                cell_fetch(P, R, k < nvalid_next, st_next.near, st_next.pbx, st_next.pby, st_next.ib,
-                           st_next.mip, c_next);
+                nvalid_next = dda_chunk(P, W, k, st);
+                c_next = cell_of_step(P, R, k < nvalid_next, st);
             }
-
-            // a cell ends where the next lane's begins
+            c.ex = entry.x;
+            c.ey = entry.y;
+            // a cell ends where the next one begins
             const float far = __shfl_sync(kWarp, k == 0 ? c_next.near : c.near, (k + 1) % kLanes);
 
             if constexpr (kCount) {
@@ -1202,10 +1209,9 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
                     const int src = __ffs(todo) - 1;
                     cnt.cells++;
                     merge_cell<true>(P, R, mask, k, row, drow, hrow, cell_of(c, src),
-                                        edge_of(edge, src), ymin, ymax, pend, cnt);
+                                        edge_of(edge, src), ymin, ymax, cnt);
                 }
             } else {
-                // ---- 2. each lane: its cell, unless it lies below the horizon ----
                 const bool alive = cell_alive(P, hz, c, far);
                 if (__ballot_sync(kWarp, alive)) {
                     const Edge edge = cell_edge(P, R, c.near, far);
@@ -1214,7 +1220,7 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
                     if (alive) nrec = scan_runs(P, R, mask, ymin, ymax, c, edge, my_recs, blockDim.x);
                     // ---- 3. the recorded runs, in the order of the walk ----
                     merge_chunk(P, R, mask, k, row, drow, hrow, c, edge, nrec, warp_recs, blockDim.x, list,
-                                   ymin, ymax, pend, q, cnt);
+                                   ymin, ymax, q, cnt);
                     if (ymin != before) hz = horizon_bound(P, R, ymin);
                 }
             }
@@ -1227,18 +1233,11 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
                 const float t_end = __shfl_sync(kWarp, far, kLanes - 1);
                 if (__fmaf_rn(hz.a, t_end, hz.scene) < 0.0f) break;
             }
-            // staging depth >= 2: the next chunk's table entries have arrived
-            // under the merge; stage each cell's header line (second header
-            // on; the first travels in the table entry) for its scan, which
-            // follows the next DDA chunk
-            if (kStage && (c_next.ey & 0xffffu) > 1u)
-                stage_headers(P.slabs[c_next.mip] + 3 + c_next.ex, staging);
             c = c_next;
             nvalid = nvalid_next;
         }
     }
-    flush_spans(P, R, q, k, row, drow, hrow, pend);
-    pend.flush();
+    if (q.n > 0) flush_spans(P, R.pos3d_z_add, R.pos3d_y_add, q.e, q.n, k, row, drow, hrow);
     __syncwarp();
 
     // ---- coalesced fill of the samples no span coloured ----
@@ -1266,19 +1265,19 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
 }
 
 // Shared memory of a raycast block: the warps' occupancy masks (`words` each,
-// padded to 16 bytes), then per thread kRecs run records, the span
-// queues (one entry per lane) and the merge's entry list (one word per lane).
+// padded to 16 bytes), their span queues (one entry per lane), the merge's
+// entry lists (one word per lane) and kRecs run records per thread.
 __host__ __device__ __forceinline__ int mask_region_words(int slots, int words) {
     return (slots * words + 3) & ~3;
 }
 __host__ __device__ __forceinline__ size_t raycast_smem_bytes(int threads, int slots, int words) {
     return static_cast<size_t>(mask_region_words(slots, words)) * 4 +
-           static_cast<size_t>(threads) * (kRecs * sizeof(uint4) + kQueueVecs * sizeof(uint4) + sizeof(uint32_t));
+           static_cast<size_t>(threads) * (kRecs * 3 * sizeof(uint32_t) + kQueueVecs * sizeof(uint4) + sizeof(uint32_t));
 }
 struct BlockSmem {
     int k, slots, slot;  // lane, warps of the block, this warp
     uint32_t* mask;      // this warp's mask
-    uint4* recs;
+    uint32_t* recs;
     uint4* spans;        // this warp's queue
     uint32_t* list;      // this warp's list
     __device__ __forceinline__ BlockSmem(uint32_t* smem, int words) {
@@ -1286,17 +1285,17 @@ struct BlockSmem {
         slots = blockDim.x / kLanes;
         slot = threadIdx.x / kLanes;
         mask = smem + slot * words;
-        recs = reinterpret_cast<uint4*>(smem + mask_region_words(slots, words));
-        uint4* queues = recs + blockDim.x * kRecs;
+        uint4* queues = reinterpret_cast<uint4*>(smem + mask_region_words(slots, words));
         spans = queues + slot * (kQueueVecs * kLanes);
-        list = reinterpret_cast<uint32_t*>(queues + blockDim.x * kQueueVecs) + slot * kLanes;
+        uint32_t* lists = reinterpret_cast<uint32_t*>(queues + blockDim.x * kQueueVecs);
+        list = lists + slot * kLanes;
+        recs = lists + blockDim.x;
     }
 };
 
 // One frame: ray slot s of block b casts ray b * slots + s.  kCount: the
-// DETAIL_BENCH counters (exact walk of every cell); kHits: hit records;
-// kStage: run-header staging (depth 2/3).
-template <bool kCount, bool kHits, bool kStage>
+// DETAIL_BENCH counters (exact walk of every cell); kHits: hit records.
+template <bool kCount, bool kHits>
 __global__ void __launch_bounds__(128, 4) raycast_kernel(const __grid_constant__ RayParams P) {
     extern __shared__ uint32_t smem[];
     const BlockSmem B(smem, (P.S + 31) >> 5);
@@ -1309,7 +1308,7 @@ __global__ void __launch_bounds__(128, 4) raycast_kernel(const __grid_constant__
         t->start_ns = global_ns();
         t->start_clock = static_cast<uint64_t>(clock64());
     }
-    cast_ray<kCount, kHits, kStage>(P, x, x < P.rays, B.mask, B.recs, B.spans, B.list, B.k, P.staging, cnt);
+    cast_ray<kCount, kHits>(P, x, x < P.rays, B.mask, B.recs, B.spans, B.list, B.k, cnt);
     if (P.ray_time && B.k == 0 && x < P.rays) {
         rle_ray_time* t = P.ray_time + x;
         t->end_clock = static_cast<uint64_t>(clock64());
@@ -1323,10 +1322,10 @@ __global__ void __launch_bounds__(128, 4) raycast_kernel(const __grid_constant__
 // index space (ray_start[f] = first global ray of frame f); each warp takes
 // `tile` consecutive rays at a time from a global counter until none are
 // left, so long and short rays of every frame balance across the GPU.
-template <bool kHits, bool kStage>
+template <bool kHits>
 __global__ void __launch_bounds__(128, 4) raycast_batch_kernel(BatchHeader* hdr, const int* __restrict__ ray_start,
-                                                            const RayParams* __restrict__ frames, int tile,
-                                                            int staging, int max_words) {
+                                                               const RayParams* __restrict__ frames, int tile,
+                                                               int max_words) {
     extern __shared__ uint32_t smem[];
     const BlockSmem B(smem, max_words);
     const int nframes = hdr->nframes;
@@ -1359,13 +1358,12 @@ __global__ void __launch_bounds__(128, 4) raycast_batch_kernel(BatchHeader* hdr,
                 }
                 f = lo;
             }
-            cast_ray<false, kHits, kStage>(frames[f], r - ray_start[f], true, B.mask, B.recs, B.spans, B.list, B.k,
-                                           staging, cnt);
+            cast_ray<false, kHits>(frames[f], r - ray_start[f], true, B.mask, B.recs, B.spans, B.list, B.k, cnt);
         }
     }
 }
 
-template <bool kCount, bool kHits, bool kStage>
+template <bool kCount, bool kHits>
 rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) {
     const int words = (p.S + 31) >> 5;
     const int rays_per_block = threads / kLanes;
@@ -1374,14 +1372,14 @@ rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) 
         set_error("rle_render_rays: %d samples per ray exceed shared memory at this launch shape", p.S);
         return RLE_ERR_CAPACITY;
     }
-    cudaError_t e = cudaFuncSetAttribute(raycast_kernel<kCount, kHits, kStage>,
+    cudaError_t e = cudaFuncSetAttribute(raycast_kernel<kCount, kHits>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) {
         set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         return RLE_ERR_CUDA;
     }
     const int blocks = (p.rays + rays_per_block - 1) / rays_per_block;
-    raycast_kernel<kCount, kHits, kStage><<<blocks, threads, smem, stream>>>(p);
+    raycast_kernel<kCount, kHits><<<blocks, threads, smem, stream>>>(p);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("raycast launch: %s", cudaGetErrorString(e));
@@ -1390,38 +1388,30 @@ rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) 
     return RLE_OK;
 }
 
-template <bool kStage>
-rle_status launch_output(const RayParams& p, int threads, cudaStream_t stream) {
-    return p.rayhit ? launch_variant<false, true, kStage>(p, threads, stream)
-                    : launch_variant<false, false, kStage>(p, threads, stream);
-}
-
 rle_status launch_shape(const RayParams& p, int threads, cudaStream_t stream) {
-    if (p.counters) {  // the counts do not depend on the staging depth
-        return p.rayhit ? launch_variant<true, true, false>(p, threads, stream)
-                        : launch_variant<true, false, false>(p, threads, stream);
-    }
-    return p.staging >= 2 ? launch_output<true>(p, threads, stream) : launch_output<false>(p, threads, stream);
+    if (p.counters)
+        return p.rayhit ? launch_variant<true, true>(p, threads, stream) : launch_variant<true, false>(p, threads, stream);
+    return p.rayhit ? launch_variant<false, true>(p, threads, stream) : launch_variant<false, false>(p, threads, stream);
 }
 
 size_t batch_smem(int threads, int max_samples) {
     return raycast_smem_bytes(threads, threads / kLanes, (max_samples + 31) >> 5);
 }
 
-template <bool kHits, bool kStage>
+template <bool kHits>
 rle_status batch_blocks(int threads, int max_samples, int* blocks) {
     const size_t smem = batch_smem(threads, max_samples);
     if (smem > 227 * 1024) {
         set_error("batch: %d samples per ray exceed shared memory at this launch shape", max_samples);
         return RLE_ERR_CAPACITY;
     }
-    cudaError_t e = cudaFuncSetAttribute(raycast_batch_kernel<kHits, kStage>,
+    cudaError_t e = cudaFuncSetAttribute(raycast_batch_kernel<kHits>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     int dev = 0, sms = 0, per_sm = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raycast_batch_kernel<kHits, kStage>,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raycast_batch_kernel<kHits>,
                                                           threads, smem);
     if (e != cudaSuccess) {
         set_error("batch launch set-up: %s", cudaGetErrorString(e));
@@ -1431,16 +1421,16 @@ rle_status batch_blocks(int threads, int max_samples, int* blocks) {
     return RLE_OK;
 }
 
-template <bool kHits, bool kStage>
+template <bool kHits>
 rle_status batch_launch(const BatchRaycast& b, cudaStream_t stream) {
     const size_t smem = batch_smem(b.threads, b.max_samples);
     int blocks = b.blocks;
     if (blocks <= 0) {
-        const rle_status st = batch_blocks<kHits, kStage>(b.threads, b.max_samples, &blocks);
+        const rle_status st = batch_blocks<kHits>(b.threads, b.max_samples, &blocks);
         if (st != RLE_OK) return st;
     }
-    raycast_batch_kernel<kHits, kStage><<<blocks, b.threads, smem, stream>>>(
-        b.header, b.ray_start, b.frames, b.tile, b.staging, (b.max_samples + 31) >> 5);
+    raycast_batch_kernel<kHits><<<blocks, b.threads, smem, stream>>>(
+        b.header, b.ray_start, b.frames, b.tile, (b.max_samples + 31) >> 5);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("batch raycast launch: %s", cudaGetErrorString(e));
@@ -1449,32 +1439,19 @@ rle_status batch_launch(const BatchRaycast& b, cudaStream_t stream) {
     return RLE_OK;
 }
 
-rle_status batch_blocks_for(int threads, int max_samples, bool hits, bool stage, int* blocks) {
-    if (stage)
-        return hits ? batch_blocks<true, true>(threads, max_samples, blocks)
-                    : batch_blocks<false, true>(threads, max_samples, blocks);
-    return hits ? batch_blocks<true, false>(threads, max_samples, blocks)
-                : batch_blocks<false, false>(threads, max_samples, blocks);
-}
-
-rle_status batch_launch_for(const BatchRaycast& b, cudaStream_t s) {
-    if (b.staging >= 2)
-        return b.hits ? batch_launch<true, true>(b, s) : batch_launch<false, true>(b, s);
-    return b.hits ? batch_launch<true, false>(b, s) : batch_launch<false, false>(b, s);
-}
-
 }  // namespace
 
-rle_status batch_grid_blocks(int threads, int max_samples, bool hits, int staging, int* blocks) {
-    return batch_blocks_for(threads, max_samples, hits, staging >= 2, blocks);
+rle_status batch_grid_blocks(int threads, int max_samples, bool hits, int* blocks) {
+    return hits ? batch_blocks<true>(threads, max_samples, blocks) : batch_blocks<false>(threads, max_samples, blocks);
 }
 
 rle_status launch_raycast_batch(const BatchRaycast& b, void* stream) {
-    if (b.threads % 32 != 0 || b.threads <= 0 || b.threads > 128 || b.tile < 1 || b.staging < 1 || b.staging > 3) {
-        set_error("batch: threads per block a multiple of 32 up to 128, tile >= 1, staging 1..3");
+    if (b.threads % 32 != 0 || b.threads <= 0 || b.threads > 128 || b.tile < 1) {
+        set_error("batch: threads per block a multiple of 32 up to 128, tile >= 1");
         return RLE_ERR_INVALID_ARG;
     }
-    return batch_launch_for(b, static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    return b.hits ? batch_launch<true>(b, s) : batch_launch<false>(b, s);
 }
 
 bool bounds_render(unsigned* out4, bool clear) {
@@ -1498,10 +1475,6 @@ rle_status launch_raycast(const RayParams& p, void* stream) {
     const int threads = p.threads_per_block > 0 ? p.threads_per_block : 128;
     if (threads % 32 != 0 || threads > 128) {
         set_error("raycast: threads per block must be a multiple of 32, at most 128");
-        return RLE_ERR_INVALID_ARG;
-    }
-    if (p.staging < 0 || p.staging > 3) {
-        set_error("raycast: staging depth 1..3 (0 = default)");
         return RLE_ERR_INVALID_ARG;
     }
     return launch_shape(p, threads, s);

@@ -105,7 +105,6 @@ struct RayParams {
     rle_counters* counters;
     rle_ray_time* ray_time;       // per-ray start/end times (single-frame kernel), or null
     int threads_per_block;        // block size (0 = default)
-    int staging;                  // staging depth of the column data (1..3; 0 = default)
 };
 
 // Per-frame constants of the resolve (uniforms of colorize_buddha_soft.frag).
@@ -146,7 +145,6 @@ struct BatchRaycast {
     const int* ray_start;      // device array [nframes + 1], prefix of rays
     const RayParams* frames;   // device array [nframes]
     int tile;                  // most adjacent rays a warp claims at once
-    int staging;               // staging depth of the column data (1..3)
     int threads;               // block size
     int max_samples;           // largest S of the frames the launch may see
     int blocks;                // grid size (0: fill the GPU)
@@ -170,7 +168,7 @@ rle_status batch_render_scenes(rle_batch* b, const rle_scene* const* scenes, con
                                void* stream, cudaEvent_t* frame_done = nullptr);
 size_t batch_capacity_words(const rle_batch* b);
 int batch_max_frames(const rle_batch* b);
-rle_status batch_grid_blocks(int threads, int max_samples, bool hits, int staging, int* blocks);
+rle_status batch_grid_blocks(int threads, int max_samples, bool hits, int* blocks);
 
 // Bounds-check words of the device code (zeros when none fired); false in
 // builds without RLE_BOUNDS_CHECK.  read: flags, first index hit; clear

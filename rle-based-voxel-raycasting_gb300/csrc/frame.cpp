@@ -85,20 +85,21 @@ rle_status fill_resolve_params(const rle_raymap* rm, ResolveParams* p) {
     }
     const float resx = static_cast<float>(rm->width), resy = static_cast<float>(rm->height);
     const float rcr = static_cast<float>(4 * rm->maxres);  // RAYS_CASTED_RES
-    p->resx = resx;
-    p->resy = resy;
+    p->geo.resx = resx;
+    p->geo.resy = resy;
     // uniforms of the colorize shader (src/main.cpp:575-603)
-    p->vanish_x = 1 - rm->vanishing_point_2d[0];
-    p->vanish_y = (1 - rm->vanishing_point_2d[1] - rm->border) * resx / resy;
+    p->geo.vanish_x = 1 - rm->vanishing_point_2d[0];
+    p->geo.vanish_y = (1 - rm->vanishing_point_2d[1] - rm->border) * resx / resy;
     const float ofs1 = 4 * static_cast<float>(rm->res[0]) / rcr;
     const float ofs2 = 4 * static_cast<float>(rm->res[1]) / rcr + ofs1;
     const float ofs3 = 4 * static_cast<float>(rm->res[2]) / rcr + ofs2;
-    p->ofs_x = -rm->p_ofs_min[0];
-    p->ofs_y = -rm->p_ofs_min[1] + ofs1;
-    p->ofs_z = -rm->p_ofs_min[2] + ofs2;
-    p->ofs_w = -rm->p_ofs_min[3] + ofs3;
-    p->ratio = rcr / static_cast<float>(rm->rows);
-    p->rxg0 = rm->rotation[0] > 0 ? 1.0f : 0.0f;
+    p->geo.ofs_x = -rm->p_ofs_min[0];
+    p->geo.ofs_y = -rm->p_ofs_min[1] + ofs1;
+    p->geo.ofs_z = -rm->p_ofs_min[2] + ofs2;
+    p->geo.ofs_w = -rm->p_ofs_min[3] + ofs3;
+    p->geo.ratio = rcr / static_cast<float>(rm->rows);
+    p->geo.rxg0 = rm->rotation[0] > 0 ? 1.0f : 0.0f;
+    resolve_derive(&p->geo);
     p->width = rm->width;
     p->height = rm->height;
     p->S = rm->samples;

@@ -6,8 +6,9 @@
 // column ray through it and the sample along that ray, then fetches the
 // texel with GL_NEAREST / GL_CLAMP_TO_EDGE (src/GL_Main.cpp:152-157).  This
 // kernel does the same arithmetic, one thread per pixel, as IEEE single
-// operations in the shader's order (compiled with -fmad=false), and decodes
-// the sample: sky, no data, or an RGB565 colour with its float depth.
+// operations in the shader's order (resolve_math.h; compiled with
+// -fmad=false), and decodes the sample: sky, no data, or an RGB565 colour with
+// its float depth.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -34,11 +35,9 @@ __device__ __forceinline__ bool in_bounds(bool ok, unsigned code, unsigned long 
 __device__ __forceinline__ bool in_bounds(bool, unsigned, unsigned long long) { return true; }
 #endif
 
-__device__ __forceinline__ float step_f(float edge, float x) { return x < edge ? 0.0f : 1.0f; }
-
+// min(max((int)floor(t * size), 0), size - 1); NaN gives 0
 __device__ __forceinline__ int texel(float t, int size) {
-    int i = static_cast<int>(floorf(t * static_cast<float>(size)));
-    return min(max(i, 0), size - 1);
+    return min(max(__float2int_rd(t * static_cast<float>(size)), 0), size - 1);
 }
 
 __device__ __forceinline__ uint32_t rgb565_to_rgba8(uint32_t c) {
@@ -51,36 +50,11 @@ __device__ __forceinline__ uint32_t rgb565_to_rgba8(uint32_t c) {
 
 template <bool kHits>
 __device__ __forceinline__ void resolve_pixel(const ResolveParams& P, int col, int row) {
-    const float RESX = P.resx, RESY = P.resy;
     const float fx = static_cast<float>(col) + 0.5f;
     const float fy = static_cast<float>(P.height - 1 - row) + 0.5f;  // GL rows count from the bottom
-    const float scx = fx / RESX, scy = fy / RESY;
-    const float border = (RESX - RESY) / (RESX * 2);
-    const float scx1 = scx - P.vanish_x, scy1 = scy - P.vanish_y;
-    const float upper = step_f(scy1, 0.0f);
-    const float left = step_f(scx1, 0.0f);
-    const float ostep = step_f(fabsf(scy1) - fabsf(scx1) * RESX / RESY, 0.0f);
-    const float seg_up = (1 - upper) * (1 - ostep);
-    const float seg_dn = upper * (1 - ostep);
-    const float seg_rt = (1 - left) * ostep;
-    const float seg_lt = left * ostep;
-    const float o2 = (ostep * fx + (1 - ostep) * fy) / RESX;
-    const float ang2 = scx1 * fabsf(1 - step_f(scy1, 0.0f) - P.vanish_y) / scy1 +
-                       step_f(scy1, 0.0f) * (1 - P.vanish_x) + (1 - step_f(scy1, 0.0f)) * P.vanish_x;
-    float ang3 = scy1 * fabsf(1 - step_f(scx1, 0.0f) - P.vanish_x) / scx1 +
-                 step_f(scx1, 0.0f) * (1 - P.vanish_y) + (1 - step_f(scx1, 0.0f)) * P.vanish_y;
-    ang3 = ang3 * RESY / RESX + border;
-    const float x_pre = ostep * ang3 + ang2 * (1 - ostep);
-    float ty = seg_dn * (P.ofs_y + x_pre) + seg_up * (P.ofs_x + 1.0f - x_pre) + seg_lt * (P.ofs_w + x_pre) +
-               seg_rt * (P.ofs_z + 1.0f - x_pre);
-    ty = ty * P.ratio * 0.25f;
-    const float r = P.rxg0;
-    const float seg_up_x = r * seg_up + (1.0f - r) * seg_dn;
-    const float seg_dn_x = r * seg_dn + (1.0f - r) * seg_up;
-    const float seg_rt_x = r * seg_rt + (1.0f - r) * seg_lt;
-    const float seg_lt_x = r * seg_lt + (1.0f - r) * seg_rt;
-    const float tx = seg_up_x * (o2 + border) + seg_dn_x * (1.0f - (o2 + border)) + seg_rt_x * o2 +
-                     seg_lt_x * (1.0f - o2);
+    float tx, ty;
+    if (P.geo.plain) resolve_coords(P.geo, fx, fy, &tx, &ty);
+    else resolve_coords_shader(P.geo, fx, fy, &tx, &ty);
     const int s = texel(tx, P.S);
     const int rr = texel(ty, P.rows);
     const size_t si = static_cast<size_t>(rr) * P.S + s;
@@ -111,10 +85,28 @@ __device__ __forceinline__ void resolve_pixel(const ResolveParams& P, int col, i
     }
 }
 
+// Bound by the L1 lines its gathers touch, then by its instructions.  In the up
+// and down fans the pixels of a screen row lie on as many column rays, a line
+// each, and those of a screen column are neighbours on one ray; to the sides it
+// is the other way round.  A warp takes 8x4 pixels, 4 to 8 lines per gather in
+// either (a row of 32: up to 32).  3840x2160 frames: 69 us with the shader's
+// arithmetic as it stands and rows of 128, 63 us with the terms that count
+// (resolve_math.h) and rows of 32, 46 us with 8x4 pixels per warp (4x8: 46, 16x2:
+// 47); 1920x1080: 20, 18, 13 us.
+constexpr int kTileX = 32, kTileY = 8;  // pixels of a block
+constexpr int kWarpX = 8, kWarpY = 4;   // pixels of a warp
+static_assert(kWarpX * kWarpY == 32 && kTileX % kWarpX == 0 && kTileY % kWarpY == 0, "tile");
+
+// Pixel of a block's thread within its tile.
+__device__ __forceinline__ int tile_col(int t) { return t / 32 % (kTileX / kWarpX) * kWarpX + t % kWarpX; }
+__device__ __forceinline__ int tile_row(int t) {
+    return t / 32 / (kTileX / kWarpX) * kWarpY + t % 32 / kWarpX;
+}
+
 template <bool kHits>
-__global__ void resolve_kernel(const __grid_constant__ ResolveParams P) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = blockIdx.y;
+__global__ void __launch_bounds__(kTileX * kTileY) resolve_kernel(const __grid_constant__ ResolveParams P) {
+    const int col = blockIdx.x * kTileX + tile_col(threadIdx.x);
+    const int row = blockIdx.y * kTileY + tile_row(threadIdx.x);
     if (col >= P.width || row >= P.height) return;
     resolve_pixel<kHits>(P, col, row);
 }
@@ -183,8 +175,8 @@ rle_status launch_resolve_batch(const BatchResolve& b, void* stream) {
 }
 
 rle_status launch_resolve(const ResolveParams& p, void* stream) {
-    const dim3 block(128, 1, 1);
-    const dim3 grid((p.width + 127) / 128, p.height, 1);
+    const dim3 block(kTileX * kTileY, 1, 1);
+    const dim3 grid((p.width + kTileX - 1) / kTileX, (p.height + kTileY - 1) / kTileY, 1);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (p.hit) resolve_kernel<true><<<grid, block, 0, s>>>(p);
     else resolve_kernel<false><<<grid, block, 0, s>>>(p);

@@ -4,6 +4,7 @@
 #include <cuda_runtime_api.h>
 #include <vector_types.h>
 
+#include "resolve_math.h"
 #include "scenegen_math.h"
 
 #include <cstddef>
@@ -109,11 +110,7 @@ struct RayParams {
 
 // Per-frame constants of the resolve (uniforms of colorize_buddha_soft.frag).
 struct ResolveParams {
-    float resx, resy;
-    float vanish_x, vanish_y;
-    float ofs_x, ofs_y, ofs_z, ofs_w;
-    float ratio;
-    float rxg0;
+    ResolveGeometry geo;
     int width, height;
     int S, rows;
     int rays;                     // rows >= rays were not cast: no data

@@ -29,6 +29,7 @@ constexpr int kThreads = 256;
 constexpr int kMaxWords = 16;  // sy <= 1024
 
 rle_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();  // a failed allocation must not fail the next call's launch check
     rle::set_error("%s: %s", what, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? RLE_ERR_NO_MEMORY : RLE_ERR_CUDA;
 }
@@ -204,8 +205,8 @@ __device__ __forceinline__ int next_bit(const uint64_t* s, int W, int p, bool wa
 }
 
 struct LevelStats {
-    unsigned long long heads, voxels;
-    unsigned int top;  // smallest stored j, 0xffffffff if none
+    unsigned long long heads, voxels, words;
+    unsigned int low;  // ~j of the smallest stored j, 0 if none (all zero at the start)
 };
 
 __global__ void __launch_bounds__(kThreads) surface_kernel(const uint64_t* __restrict__ cols, int sx, int sy, int sz,
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(kThreads) surface_kernel(const uint64_t* __res
     if ((threadIdx.x & 31) == 0) {
         if (heads) atomicAdd(&stats->heads, heads);
         if (voxels) atomicAdd(&stats->voxels, voxels);
-        if (top != 0xffffffffu) atomicMin(&stats->top, top);
+        if (top != 0xffffffffu) atomicMax(&stats->low, ~top);
     }
 }
 
@@ -537,23 +538,14 @@ struct DevLevel {
     uint64_t* cols = nullptr;
 };
 
+// Working buffers of the levels encoded together.
 struct Scratch {
-    uint64_t* surf = nullptr;
-    uint32_t* nwords = nullptr;
-    uint16_t* nhead = nullptr;
-    unsigned long long* offsets = nullptr;
+    uint64_t* surf[RLE_MAX_MIPS] = {};
+    uint32_t* nwords[RLE_MAX_MIPS] = {};
+    uint16_t* nhead[RLE_MAX_MIPS] = {};
+    unsigned long long* offsets[RLE_MAX_MIPS] = {};
     unsigned long long* sums = nullptr;
     LevelStats* stats = nullptr;  // device, one per level
-    unsigned long long* total = nullptr;
-    void release() {
-        cudaFree(surf);
-        cudaFree(nwords);
-        cudaFree(nhead);
-        cudaFree(offsets);
-        cudaFree(sums);
-        cudaFree(stats);
-        cudaFree(total);
-    }
 };
 
 struct Build {
@@ -561,9 +553,12 @@ struct Build {
     cudaStream_t stream = nullptr;
     std::vector<DevLevel> lv;
     Scratch sc;
+    int group = 0;          // levels encoded together
+    void* block = nullptr;  // the levels, the scratch of one and the totals
+    void* extra = nullptr;  // the scratch of the others, where they are encoded together
     ~Build() {
-        for (DevLevel& l : lv) cudaFree(l.cols);
-        sc.release();
+        if (extra) cudaFree(extra);
+        if (block) cudaFree(block);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -573,6 +568,41 @@ rle_status launch_check(const char* what) {
     return e == cudaSuccess ? RLE_OK : cuda_fail(e, what);
 }
 
+struct Carve {
+    char* at;  // null: counts only
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, size_t n) {
+        p = at ? reinterpret_cast<T*>(at + used) : nullptr;
+        used += (n * sizeof(T) + 255) & ~static_cast<size_t>(255);
+    }
+};
+
+// Scratch of level m in slot m; slot 0 also serves the levels that are
+// encoded one by one, none larger than level 0.
+void lay_out_slot(Build& B, int m, Carve& c) {
+    const DevLevel& L = B.lv[m];
+    const size_t n = static_cast<size_t>(L.sx) * L.sz;
+    c.take(B.sc.surf[m], n * L.W);
+    c.take(B.sc.nwords[m], n);
+    c.take(B.sc.nhead[m], n);
+    c.take(B.sc.offsets[m], n);
+}
+
+void lay_out_block(Build& B, Carve& c) {
+    for (DevLevel& L : B.lv) c.take(L.cols, static_cast<size_t>(L.sx) * L.sz * L.W);
+    lay_out_slot(B, 0, c);
+    c.take(B.sc.sums, (static_cast<size_t>(B.lv[0].sx) * B.lv[0].sz + kScanChunk - 1) / kScanChunk);
+    c.take(B.sc.stats, RLE_MAX_MIPS);
+}
+
+void lay_out_extra(Build& B, Carve& c) {
+    for (size_t m = 1; m < B.lv.size(); m++) lay_out_slot(B, static_cast<int>(m), c);
+}
+
+// Two allocations for the build.  The levels are encoded together, so that the
+// host waits for their sizes once; where the scratch of all of them does not
+// fit the device, one by one with the scratch of the largest.
 rle_status alloc_levels(Build& B, int sx, int sy, int sz, int nummaps) {
     B.lv.resize(nummaps);
     for (int m = 0; m < nummaps; m++) {
@@ -581,21 +611,28 @@ rle_status alloc_levels(Build& B, int sx, int sy, int sz, int nummaps) {
         L.sz = sz >> m;
         L.sy = m == 0 ? sy : B.lv[m - 1].sy / 2;
         L.W = (L.sy + 63) / 64;
-        const size_t bytes = static_cast<size_t>(L.sx) * L.sz * L.W * 8;
-        const cudaError_t e = cudaMalloc(&L.cols, bytes);
-        if (e != cudaSuccess) return cuda_fail(e, "scene build: cudaMalloc(level bits)");
     }
-    const long long n0 = static_cast<long long>(sx) * sz;
-    const long long nb = (n0 + kScanChunk - 1) / kScanChunk;
-    cudaError_t e;
-    if ((e = cudaMalloc(&B.sc.surf, static_cast<size_t>(n0) * B.lv[0].W * 8)) != cudaSuccess ||
-        (e = cudaMalloc(&B.sc.nwords, static_cast<size_t>(n0) * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&B.sc.nhead, static_cast<size_t>(n0) * 2)) != cudaSuccess ||
-        (e = cudaMalloc(&B.sc.offsets, static_cast<size_t>(n0) * 8)) != cudaSuccess ||
-        (e = cudaMalloc(&B.sc.sums, static_cast<size_t>(nb) * 8)) != cudaSuccess ||
-        (e = cudaMalloc(&B.sc.stats, sizeof(LevelStats) * RLE_MAX_MIPS)) != cudaSuccess ||
-        (e = cudaMalloc(&B.sc.total, 8)) != cudaSuccess)
-        return cuda_fail(e, "scene build: cudaMalloc(scratch)");
+    Carve count{nullptr};
+    lay_out_block(B, count);
+    const cudaError_t e = cudaMalloc(&B.block, count.used);
+    if (e != cudaSuccess) {
+        B.block = nullptr;
+        return cuda_fail(e, "scene build: cudaMalloc(working buffers)");
+    }
+    Carve block{static_cast<char*>(B.block)};
+    lay_out_block(B, block);
+    B.group = 1;
+    if (nummaps == 1) return RLE_OK;
+    Carve more{nullptr};
+    lay_out_extra(B, more);
+    if (cudaMalloc(&B.extra, more.used) != cudaSuccess) {
+        cudaGetLastError();
+        B.extra = nullptr;
+        return RLE_OK;
+    }
+    Carve extra{static_cast<char*>(B.extra)};
+    lay_out_extra(B, extra);
+    B.group = nummaps;
     return RLE_OK;
 }
 
@@ -611,95 +648,115 @@ rle_status build_mips(Build& B) {
     return RLE_OK;
 }
 
-// Encodes every level into a new scene.
-rle_status encode_levels(Build& B, WriteArgs base, rle_scene** out) {
+// Surface, counts and offsets of level m into scratch slot i.
+rle_status count_level(Build& B, int m, int i) {
+    const DevLevel& L = B.lv[m];
+    const long long n = static_cast<long long>(L.sx) * L.sz;
+    const long long nb = (n + kScanChunk - 1) / kScanChunk;
+    Scratch& sc = B.sc;
+    rle_status st;
+    surface_kernel<<<grid_for(n), kThreads, 0, B.stream>>>(L.cols, L.sx, L.sy, L.sz, L.W, sc.surf[i], sc.nwords[i],
+                                                            sc.nhead[i], sc.stats + m);
+    if ((st = launch_check("surface_kernel")) != RLE_OK) return st;
+    scan_reduce_kernel<<<static_cast<unsigned>(nb), kScanThreads, 0, B.stream>>>(sc.nwords[i], n, sc.sums);
+    if ((st = launch_check("scan_reduce_kernel")) != RLE_OK) return st;
+    scan_sums_kernel<<<1, kScanThreads, 0, B.stream>>>(sc.sums, nb, &sc.stats[m].words);
+    if ((st = launch_check("scan_sums_kernel")) != RLE_OK) return st;
+    scan_down_kernel<<<static_cast<unsigned>(nb), kScanThreads, 0, B.stream>>>(sc.nwords[i], n, sc.sums,
+                                                                                sc.offsets[i]);
+    return launch_check("scan_down_kernel");
+}
+
+// Words of level m (counted in slot i) into the scene's level.
+rle_status write_level(Build& B, const WriteArgs& base, rle::Level& D, int m, int i) {
+    const DevLevel& L = B.lv[m];
+    // zero padding after the words (the writer covers every word)
+    const cudaError_t e =
+        cudaMemsetAsync(reinterpret_cast<char*>(D.d_slabs) + D.words * 2, 0, rle::kSlabPadBytes, B.stream);
+    if (e != cudaSuccess) return cuda_fail(e, "scene build: cudaMemsetAsync(padding)");
+    WriteArgs a = base;
+    a.cols = L.cols;
+    a.mip = m;
+    a.sx = L.sx;
+    a.sy = L.sy;
+    a.sz = L.sz;
+    a.W = L.W;
+    a.words = D.words;
+    write_kernel<<<grid_for(static_cast<long long>(L.sx) * L.sz), kThreads, 0, B.stream>>>(
+        a, B.sc.surf[i], B.sc.offsets[i], B.sc.nhead[i], D.d_slabs, reinterpret_cast<uint2*>(D.d_table));
+    return launch_check("write_kernel");
+}
+
+// Encodes every level into the scene, B.group levels at a time.
+rle_status encode_into(Build& B, const WriteArgs& base, rle_scene* s) {
     const int nummaps = static_cast<int>(B.lv.size());
     cudaError_t e = cudaMemsetAsync(B.sc.stats, 0, sizeof(LevelStats) * RLE_MAX_MIPS, B.stream);
     if (e != cudaSuccess) return cuda_fail(e, "scene build: cudaMemsetAsync");
-    std::vector<LevelStats> init(RLE_MAX_MIPS);
-    for (auto& s : init) s = LevelStats{0, 0, 0xffffffffu};
-    e = cudaMemcpyAsync(B.sc.stats, init.data(), sizeof(LevelStats) * RLE_MAX_MIPS, cudaMemcpyHostToDevice, B.stream);
-    if (e != cudaSuccess) return cuda_fail(e, "scene build: stats upload");
-    e = cudaStreamSynchronize(B.stream);
-    if (e != cudaSuccess) return cuda_fail(e, "scene build");
+    long long top_all = 0x7fffffffLL;
+    LevelStats stats[RLE_MAX_MIPS];
+    for (int m0 = 0; m0 < nummaps; m0 += B.group) {
+        const int m1 = m0 + B.group < nummaps ? m0 + B.group : nummaps;
+        rle_status st;
+        for (int m = m0; m < m1; m++)
+            if ((st = count_level(B, m, m - m0)) != RLE_OK) return st;
+        if ((e = cudaMemcpyAsync(stats, B.sc.stats, sizeof(stats), cudaMemcpyDeviceToHost, B.stream)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(B.stream)) != cudaSuccess)
+            return cuda_fail(e, "scene build: level totals");
+        for (int m = m0; m < m1; m++) {
+            const LevelStats& ls = stats[m];
+            if (ls.words > 0xffffffffull) {
+                rle::set_error("scene build: level %d needs %llu slab words (the column table holds 32-bit offsets)",
+                               m, ls.words);
+                return RLE_ERR_CAPACITY;
+            }
+            rle::Level& D = s->lv[m];
+            D.sx = B.lv[m].sx;
+            D.sy = B.lv[m].sy;
+            D.sz = B.lv[m].sz;
+            D.words = ls.words;
+            s->device_bytes += static_cast<size_t>(D.sx) * D.sz * 8 + static_cast<size_t>(D.words) * 2 +
+                               rle::kSlabPadBytes;
+            if (m == 0) {
+                s->run_headers = ls.heads;
+                s->surface_voxels = ls.voxels;
+            }
+            // same clamp as the loader: an empty level reports INT_MAX
+            const unsigned int low = ~ls.low;
+            const int top = low > 0x7fffffffu ? 0x7fffffff : static_cast<int>(low);
+            const long long top0 = static_cast<long long>(top) << m;
+            if (top0 < top_all) top_all = top0;
+        }
+        if ((e = rle::alloc_scene_levels(s, m0, m1)) != cudaSuccess) {
+            if (e != cudaErrorMemoryAllocation || B.group == 1)
+                return cuda_fail(e, "scene build: cudaMalloc(tables and slabs)");
+            // no room beside the scratch of all levels: again, one by one
+            cudaGetLastError();
+            cudaFree(B.extra);
+            B.extra = nullptr;
+            B.group = 1;
+            s->device_bytes = 0;
+            return encode_into(B, base, s);
+        }
+        for (int m = m0; m < m1; m++)
+            if ((st = write_level(B, base, s->lv[m], m, m - m0)) != RLE_OK) return st;
+    }
+    if ((e = cudaStreamSynchronize(B.stream)) != cudaSuccess) return cuda_fail(e, "scene build");
+    s->top_index = static_cast<int>(top_all);
+    return RLE_OK;
+}
 
+rle_status encode_levels(Build& B, const WriteArgs& base, rle_scene** out) {
     rle_scene* s = new (std::nothrow) rle_scene();
     if (!s) return RLE_ERR_NO_MEMORY;
     s->device = B.device;
-    s->nummaps = nummaps;
+    s->nummaps = static_cast<int>(B.lv.size());
     s->height = B.lv[0].sy;
-    long long top_all = 0x7fffffffLL;
-    rle_status st = RLE_OK;
-    for (int m = 0; m < nummaps && st == RLE_OK; m++) {
-        const DevLevel& L = B.lv[m];
-        const long long n = static_cast<long long>(L.sx) * L.sz;
-        const long long nb = (n + kScanChunk - 1) / kScanChunk;
-        surface_kernel<<<grid_for(n), kThreads, 0, B.stream>>>(L.cols, L.sx, L.sy, L.sz, L.W, B.sc.surf,
-                                                                B.sc.nwords, B.sc.nhead, B.sc.stats + m);
-        if ((st = launch_check("surface_kernel")) != RLE_OK) break;
-        scan_reduce_kernel<<<static_cast<unsigned>(nb), kScanThreads, 0, B.stream>>>(B.sc.nwords, n, B.sc.sums);
-        if ((st = launch_check("scan_reduce_kernel")) != RLE_OK) break;
-        scan_sums_kernel<<<1, kScanThreads, 0, B.stream>>>(B.sc.sums, nb, B.sc.total);
-        if ((st = launch_check("scan_sums_kernel")) != RLE_OK) break;
-        scan_down_kernel<<<static_cast<unsigned>(nb), kScanThreads, 0, B.stream>>>(B.sc.nwords, n, B.sc.sums,
-                                                                                    B.sc.offsets);
-        if ((st = launch_check("scan_down_kernel")) != RLE_OK) break;
-        unsigned long long words = 0;
-        LevelStats ls;
-        if ((e = cudaMemcpyAsync(&words, B.sc.total, 8, cudaMemcpyDeviceToHost, B.stream)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(&ls, B.sc.stats + m, sizeof(ls), cudaMemcpyDeviceToHost, B.stream)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(B.stream)) != cudaSuccess) {
-            st = cuda_fail(e, "scene build: level totals");
-            break;
-        }
-        if (words > 0xffffffffull) {
-            rle::set_error("scene build: level %d needs %llu slab words (the column table holds 32-bit offsets)", m,
-                           words);
-            st = RLE_ERR_CAPACITY;
-            break;
-        }
-        rle::Level& D = s->lv[m];
-        D.sx = L.sx;
-        D.sy = L.sy;
-        D.sz = L.sz;
-        D.words = words;
-        const size_t tbytes = static_cast<size_t>(n) * 8;
-        const size_t sbytes = static_cast<size_t>(words) * 2 + rle::kSlabPadBytes;
-        if ((e = cudaMalloc(&D.d_table, tbytes)) != cudaSuccess) { st = cuda_fail(e, "scene build: cudaMalloc(table)"); break; }
-        if ((e = cudaMalloc(&D.d_slabs, sbytes)) != cudaSuccess) { st = cuda_fail(e, "scene build: cudaMalloc(slabs)"); break; }
-        // zero padding after the words (the writer covers every word)
-        if ((e = cudaMemsetAsync(reinterpret_cast<char*>(D.d_slabs) + words * 2, 0, rle::kSlabPadBytes, B.stream)) !=
-            cudaSuccess) {
-            st = cuda_fail(e, "scene build: cudaMemsetAsync(padding)");
-            break;
-        }
-        s->device_bytes += tbytes + sbytes;
-        WriteArgs a = base;
-        a.cols = L.cols;
-        a.mip = m;
-        a.sx = L.sx;
-        a.sy = L.sy;
-        a.sz = L.sz;
-        a.W = L.W;
-        a.words = words;
-        write_kernel<<<grid_for(n), kThreads, 0, B.stream>>>(a, B.sc.surf, B.sc.offsets, B.sc.nhead, D.d_slabs,
-                                                             reinterpret_cast<uint2*>(D.d_table));
-        if ((st = launch_check("write_kernel")) != RLE_OK) break;
-        if (m == 0) {
-            s->run_headers = ls.heads;
-            s->surface_voxels = ls.voxels;
-        }
-        // same clamp as the loader: an empty level reports INT_MAX
-        const int top = ls.top > 0x7fffffffu ? 0x7fffffff : static_cast<int>(ls.top);
-        const long long top0 = static_cast<long long>(top) << m;
-        if (top0 < top_all) top_all = top0;
-    }
-    if (st == RLE_OK && (e = cudaStreamSynchronize(B.stream)) != cudaSuccess) st = cuda_fail(e, "scene build");
+    const rle_status st = encode_into(B, base, s);
     if (st != RLE_OK) {
+        cudaStreamSynchronize(B.stream);  // launched writes end before their memory goes
         rle_scene_free(s);
         return st;
     }
-    s->top_index = static_cast<int>(top_all);
     *out = s;
     return RLE_OK;
 }

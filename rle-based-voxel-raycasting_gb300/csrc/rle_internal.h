@@ -27,6 +27,7 @@ struct Level {
     uint64_t words = 0;
     uint32_t* d_table = nullptr;  // 2 * sx * sz words
     uint16_t* d_slabs = nullptr;  // words (+ 8 words of zero padding)
+    void* block = nullptr;        // the allocation this level starts, if any (it may hold later levels too)
 };
 
 }  // namespace rle
@@ -54,6 +55,11 @@ constexpr size_t kSlabPadBytes = 65536;
 #else
 constexpr size_t kSlabPadBytes = 16;
 #endif
+
+// Tables and slabs of levels first .. end-1 (sizes and words set) in one
+// allocation, owned by level `first`: an allocation and its release cost the
+// host 20 to 100 us each, more than the kernels of a small level.
+cudaError_t alloc_scene_levels(rle_scene* s, int first, int end);
 
 // Bounds-check word codes (RLE_BOUNDS_CHECK builds).
 enum BoundsCode : unsigned {

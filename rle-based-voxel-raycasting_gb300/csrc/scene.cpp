@@ -157,9 +157,35 @@ rle_status build_table(const HostLevel& lv, uint32_t* table, uint64_t* run_heade
 
 }  // namespace rle
 
+namespace rle {
+
+cudaError_t alloc_scene_levels(rle_scene* s, int first, int end) {
+    auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
+    auto table_bytes = [](const Level& lv) { return static_cast<size_t>(lv.sx) * lv.sz * 8; };
+    auto slab_bytes = [](const Level& lv) { return static_cast<size_t>(lv.words) * 2 + kSlabPadBytes; };
+    size_t total = 0;
+    for (int m = first; m < end; m++) total += up(table_bytes(s->lv[m])) + up(slab_bytes(s->lv[m]));
+    void* block = nullptr;
+    const cudaError_t e = cudaMalloc(&block, total);
+    if (e != cudaSuccess) return e;
+    s->lv[first].block = block;
+    char* at = static_cast<char*>(block);
+    for (int m = first; m < end; m++) {
+        Level& lv = s->lv[m];
+        lv.d_table = reinterpret_cast<uint32_t*>(at);
+        at += up(table_bytes(lv));
+        lv.d_slabs = reinterpret_cast<uint16_t*>(at);
+        at += up(slab_bytes(lv));
+    }
+    return cudaSuccess;
+}
+
+}  // namespace rle
+
 namespace {
 
 rle_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();  // a failed allocation must not fail the next call's launch check
     rle::set_error("%s: %s", what, cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? RLE_ERR_NO_MEMORY : RLE_ERR_CUDA;
 }
@@ -170,8 +196,8 @@ void release(rle_scene* s) {
     cudaGetDevice(&prev);
     cudaSetDevice(s->device);
     for (auto& lv : s->lv) {
-        if (lv.d_table) cudaFree(lv.d_table);
-        if (lv.d_slabs) cudaFree(lv.d_slabs);
+        if (lv.block) cudaFree(lv.block);
+        lv.block = nullptr;
         lv.d_table = nullptr;
         lv.d_slabs = nullptr;
     }
@@ -239,23 +265,25 @@ extern "C" rle_status rle_scene_load_memory(const void* bytes, size_t nbytes, in
     s->top_index = static_cast<int>(top_all);
     s->height = levels[0].sy;
     s->surface_voxels = vox0;
+    for (int m = 0; m < nummaps; m++) {
+        s->lv[m].sx = levels[m].sx;
+        s->lv[m].sy = levels[m].sy;
+        s->lv[m].sz = levels[m].sz;
+        s->lv[m].words = levels[m].words;
+    }
+    e = rle::alloc_scene_levels(s, 0, nummaps);
+    if (e != cudaSuccess) st = cuda_fail(e, "cudaMalloc(scene)");
     for (int m = 0; m < nummaps && st == RLE_OK; m++) {
         const rle::HostLevel& hl = levels[m];
         rle::Level& lv = s->lv[m];
-        lv.sx = hl.sx;
-        lv.sy = hl.sy;
-        lv.sz = hl.sz;
-        lv.words = hl.words;
         const size_t cols = static_cast<size_t>(hl.sx) * hl.sz;
         const std::vector<uint32_t>& table = tables[m];
         const size_t tbytes = cols * 8;
         // 16 bytes of zero padding after the words keep 16-byte vector loads
         // of a column's last header group inside the allocation.
         const size_t sbytes = static_cast<size_t>(hl.words) * 2 + rle::kSlabPadBytes;
-        if ((e = cudaMalloc(&lv.d_table, tbytes)) != cudaSuccess) { st = cuda_fail(e, "cudaMalloc(table)"); break; }
-        if ((e = cudaMalloc(&lv.d_slabs, sbytes)) != cudaSuccess) { st = cuda_fail(e, "cudaMalloc(slabs)"); break; }
         if ((e = cudaMemcpy(lv.d_table, table.data(), tbytes, cudaMemcpyHostToDevice)) != cudaSuccess) { st = cuda_fail(e, "cudaMemcpy(table)"); break; }
-        if ((e = cudaMemset(lv.d_slabs, 0, sbytes)) != cudaSuccess) { st = cuda_fail(e, "cudaMemset(slabs)"); break; }
+        if ((e = cudaMemset(reinterpret_cast<char*>(lv.d_slabs) + (sbytes - rle::kSlabPadBytes), 0, rle::kSlabPadBytes)) != cudaSuccess) { st = cuda_fail(e, "cudaMemset(slabs)"); break; }
         if (hl.words && (e = cudaMemcpy(lv.d_slabs, hl.slabs, static_cast<size_t>(hl.words) * 2, cudaMemcpyHostToDevice)) != cudaSuccess) { st = cuda_fail(e, "cudaMemcpy(slabs)"); break; }
         s->device_bytes += tbytes + sbytes;
     }

@@ -174,7 +174,8 @@ rle_status rle_scenegen_device(const rle_scenegen_params* p, int device, rle_sce
  * d_colours[(i<<m) + (j<<m)*sx + (k<<m)*sx*sy] when d_colours is not NULL
  * (u16 per level-0 voxel, same index as the bits), else the reference's
  * normal-derived word without material bits (src/Rle4.cpp:134-161, col1 ==
- * NULL).  Reads the inputs on `device`; does not modify them. */
+ * NULL).  Reads the inputs on `device`; does not modify them.  They must be
+ * complete: the build runs on a stream of its own, which waits for no other. */
 rle_status rle_encode_device(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz,
                              int nummaps, int device, rle_scene** out);
 

@@ -2,10 +2,11 @@
 // >= 3-of-8 rule, RLE4::compress's surface rule and run-length encoding,
 // and RLE4::load's column table, as kernels over column bitsets in HBM.
 //
-// Working layout: one level as column bitsets, cols[(z*sx + x)*W + w] with
+// Working layout: one level as column bitsets, cols[(z*W + w)*sx + x] with
 // W = ceil(sy/64) u64 words per column, bit j&63 of word j>>6 being voxel j
 // of the column counted from the top (the reference's j,
-// src/Rle4.cpp:83-88).  A level is encoded in four launches:
+// src/Rle4.cpp:83-88).  Equal words of neighbouring columns are neighbours, so
+// a warp of columns reads and writes whole lines.  A level is encoded in four launches:
 //   surface_kernel  surface bits (solid with < 27 solid in-bounds
 //                   neighbours, src/Rle4.cpp:100-132) + words per column
 //   scan            exclusive prefix of the words -> slab offsets (u64)
@@ -26,7 +27,6 @@ namespace {
 using rle::gen::Consts;
 
 constexpr int kThreads = 256;
-constexpr int kMaxWords = 16;  // sy <= 1024
 
 rle_status cuda_fail(cudaError_t e, const char* what) {
     cudaGetLastError();  // a failed allocation must not fail the next call's launch check
@@ -72,14 +72,13 @@ __global__ void __launch_bounds__(kThreads) gen_columns_kernel(const __grid_cons
     const long long tile = t >> 5;
     const int x = static_cast<int>(tile & (tiles - 1)) * 8 + (lane & 7);
     const int z = static_cast<int>(tile / tiles) * 4 + (lane >> 3);
-    const long long q = static_cast<long long>(z) * c.sx + x;
     const int h = rle::gen::ground_height(c, x, z);
     int y0 = static_cast<int>(c.cave_y0), y1 = static_cast<int>(c.cave_y1);
     if (y0 < 1) y0 = 1;
     if (y1 > h) y1 = h;
     const int ground_j = c.sy - h;  // storage indices >= ground_j are solid
     const float inv = 1.0f / c.cave_period;
-    uint64_t* out = cols + q * a.W;
+    uint64_t* out = cols + static_cast<long long>(z) * a.W * c.sx + x;
     for (int w = 0; w < a.W; w++) {
         const int j0 = w * 64;
         uint64_t word;
@@ -96,7 +95,7 @@ __global__ void __launch_bounds__(kThreads) gen_columns_kernel(const __grid_cons
                 word &= ~(static_cast<uint64_t>(carve) << (j - j0));
             }
         }
-        out[w] = word;
+        out[static_cast<long long>(w) * c.sx] = word;
     }
 }
 
@@ -119,7 +118,7 @@ __global__ void __launch_bounds__(kThreads) transpose_kernel(const uint8_t* __re
         const long long idx = x + static_cast<long long>(j) * sx + z * sxy;
         word |= static_cast<uint64_t>((bits[idx >> 3] >> (x & 7)) & 1) << (j & 63);
     }
-    cols[(static_cast<long long>(z) * sx + x) * W + w] = word;
+    cols[t] = word;
 }
 
 // ----------------------------------------------------------------- mips
@@ -150,19 +149,20 @@ __global__ void __launch_bounds__(kThreads) halve_kernel(const uint64_t* __restr
     const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (q >= static_cast<long long>(bsx) * bsz) return;
     const int i = static_cast<int>(q % bsx), k = static_cast<int>(q / bsx);
-    const uint64_t* c0 = a + (static_cast<long long>(2 * k) * asx + 2 * i) * aW;
-    const uint64_t* c1 = c0 + aW;
-    const uint64_t* c2 = a + (static_cast<long long>(2 * k + 1) * asx + 2 * i) * aW;
-    const uint64_t* c3 = c2 + aW;
+    const uint64_t* r0 = a + static_cast<long long>(2 * k) * aW * asx + 2 * i;
+    const uint64_t* r1 = r0 + static_cast<long long>(aW) * asx;
     const uint64_t m55 = 0x5555555555555555ull, m33 = 0x3333333333333333ull;
-    uint64_t* dst = b + q * bW;
+    uint64_t* dst = b + static_cast<long long>(k) * bW * bsx + i;
     uint64_t acc = 0;
     int written = 0;
     for (int w = 0; w < aW; w++) {
         const int j0 = 32 * w;
         if (j0 >= bsy) break;
         uint64_t sa = 0, sb = 0;
-        const uint64_t v4[4] = {c0[w], c1[w], c2[w], c3[w]};
+        // asx is even and the levels start on 256 bytes: pairs are aligned
+        const ulonglong2 p0 = *reinterpret_cast<const ulonglong2*>(r0 + static_cast<long long>(w) * asx);
+        const ulonglong2 p1 = *reinterpret_cast<const ulonglong2*>(r1 + static_cast<long long>(w) * asx);
+        const uint64_t v4[4] = {p0.x, p0.y, p1.x, p1.y};
 #pragma unroll
         for (int t = 0; t < 4; t++) {
             const uint64_t pc = (v4[t] & m55) + ((v4[t] >> 1) & m55);  // 2-bit pair counts
@@ -174,13 +174,13 @@ __global__ void __launch_bounds__(kThreads) halve_kernel(const uint64_t* __restr
         const uint32_t bits = spread16(compact_nibble_lsbs(ga)) | (spread16(compact_nibble_lsbs(gb)) << 1);
         acc |= static_cast<uint64_t>(bits) << (j0 & 63);
         if ((j0 & 63) == 32 || w == aW - 1 || 32 * (w + 1) >= bsy) {
-            dst[j0 >> 6] = acc;
             written = (j0 >> 6) + 1;
+            if (written == bW && (bsy & 63)) acc &= (1ull << (bsy & 63)) - 1;
+            dst[static_cast<long long>(written - 1) * bsx] = acc;
             acc = 0;
         }
     }
-    for (int w = written; w < bW; w++) dst[w] = 0;
-    if (bsy & 63) dst[bW - 1] &= (1ull << (bsy & 63)) - 1;
+    for (int w = written; w < bW; w++) dst[static_cast<long long>(w) * bsx] = 0;
 }
 
 // ------------------------------------------------------- surface + count
@@ -192,62 +192,83 @@ __device__ __forceinline__ int run_headers(int skip, int solid) {
     return (skip > 0 ? (skip - 1) / 1023 : 0) + (solid - 1) / 63 + 1;
 }
 
-// First index >= p whose bit equals `want` (bits past the words read as 0).
-__device__ __forceinline__ int next_bit(const uint64_t* s, int W, int p, bool want) {
-    int w = p >> 6;
-    if (w >= W) return want ? W * 64 : p;
-    uint64_t word = (want ? s[w] : ~s[w]) & (~0ull << (p & 63));
-    while (!word) {
-        if (++w >= W) return want ? W * 64 : W * 64;
-        word = want ? s[w] : ~s[w];
-    }
-    return w * 64 + __ffsll(static_cast<long long>(word)) - 1;
-}
-
 struct LevelStats {
     unsigned long long heads, voxels, words;
     unsigned int low;  // ~j of the smallest stored j, 0 if none (all zero at the start)
 };
 
+// One thread per column, its words in order.  A voxel is interior when the
+// 3x3 columns around it are solid at its height and at the two next to it:
+// with A the AND of the nine columns, A & A << 1 & A >> 1.  A thread ANDs the
+// three columns of its x, and takes the two next to it from the neighbouring
+// lanes.  Runs are counted at the toggles of the surface bits.  Was 3 x 9
+// strided loads a word and the words in local memory: 495 -> 292 us at 2048 x
+// 2048 x 256, where the walk over the toggles bounds it now.
 __global__ void __launch_bounds__(kThreads) surface_kernel(const uint64_t* __restrict__ cols, int sx, int sy, int sz,
                                                            int W, uint64_t* __restrict__ surf,
                                                            uint32_t* __restrict__ nwords,
                                                            uint16_t* __restrict__ nhead, LevelStats* stats) {
     const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const bool valid = q < static_cast<long long>(sx) * sz;
+    const int x = static_cast<int>(q % sx), z = static_cast<int>(q / sx);
+    const bool edge = x == 0 || z == 0 || x == sx - 1 || z == sz - 1;
+    const bool inside = valid && z > 0 && z < sz - 1;  // has rows on both sides
+    const long long row = static_cast<long long>(W) * sx;
+    const uint64_t* self = cols + z * row + x;
+    // AND of the columns of x (+ dx) in the three rows, word w
+    auto three = [&](int w, int dx) {
+        const uint64_t* n = self + static_cast<long long>(w) * sx + dx;
+        return n[-row] & n[0] & n[row];
+    };
+    // the nine; every lane of the warp comes here
+    auto nine = [&](int w) {
+        uint64_t mid = 0, left, right;
+        if (inside) mid = three(w, 0);
+        left = __shfl_up_sync(0xffffffffu, mid, 1);
+        right = __shfl_down_sync(0xffffffffu, mid, 1);
+        if (inside && !edge) {
+            if (lane == 0) left = three(w, -1);
+            if (lane == 31) right = three(w, 1);
+        }
+        return mid & left & right;
+    };
     unsigned long long heads = 0, voxels = 0;
     unsigned int top = 0xffffffffu;
-    if (q < static_cast<long long>(sx) * sz) {
-        const int x = static_cast<int>(q % sx), z = static_cast<int>(q / sx);
-        const bool edge = x == 0 || z == 0 || x == sx - 1 || z == sz - 1;
-        const uint64_t* self = cols + q * W;
-        uint64_t s[kMaxWords];
-        for (int w = 0; w < W; w++) {
-            uint64_t v = self[w];
+    int nh = 0, start = 0, end = 0;
+    uint64_t before = 0, open = 0;  // the word before's nine; whether its last bit was set
+    uint64_t here = nine(0);
+    for (int w = 0; w < W; w++) {
+        const uint64_t after = w + 1 < W ? nine(w + 1) : 0;
+        if (valid) {
+            uint64_t v = self[static_cast<long long>(w) * sx];
             if (!edge) {
-                uint64_t inner = ~0ull;
-                for (int dz = -1; dz <= 1; dz++)
-                    for (int dx = -1; dx <= 1; dx++) {
-                        const uint64_t* n = cols + ((static_cast<long long>(z) + dz) * sx + x + dx) * W;
-                        const uint64_t below = (n[w] << 1) | (w > 0 ? n[w - 1] >> 63 : 0);      // bit j = n[j-1]
-                        const uint64_t above = (n[w] >> 1) | (w + 1 < W ? n[w + 1] << 63 : 0);  // bit j = n[j+1]
-                        inner &= n[w] & below & above;
-                    }
+                uint64_t inner = here & ((here << 1) | (before >> 63)) & ((here >> 1) | (after << 63));
                 // j = 0 and j = sy-1 have an out-of-bounds neighbour: never interior
                 if (w == 0) inner &= ~1ull;
                 if (w == ((sy - 1) >> 6)) inner &= ~(1ull << ((sy - 1) & 63));
                 v &= ~inner;
             }
-            s[w] = v;
-            surf[q * W + w] = v;
+            surf[z * row + static_cast<long long>(w) * sx + x] = v;
             voxels += __popcll(v);
+            for (uint64_t t = v ^ ((v << 1) | open); t; t &= t - 1) {
+                const int at = w * 64 + __ffsll(static_cast<long long>(t)) - 1;
+                open ^= 1;
+                if (open) {
+                    if (top == 0xffffffffu) top = static_cast<unsigned>(at);
+                    start = at;
+                } else {
+                    nh += run_headers(start - end, at - start);
+                    end = at;
+                }
+            }
+            open = v >> 63;
         }
-        int nh = 0, end = 0;
-        for (int a = next_bit(s, W, 0, true); a < sy; a = next_bit(s, W, end, true)) {
-            const int b = next_bit(s, W, a, false);
-            if (top == 0xffffffffu) top = static_cast<unsigned>(a);
-            nh += run_headers(a - end, b - a);
-            end = b;
-        }
+        before = here;
+        here = after;
+    }
+    if (valid) {
+        if (open) nh += run_headers(start - end, W * 64 - start);
         heads = static_cast<unsigned long long>(nh);
         nwords[q] = static_cast<uint32_t>(2 + nh + voxels);
         nhead[q] = static_cast<uint16_t>(nh);
@@ -363,6 +384,10 @@ struct WriteArgs {
     int mode, mip;
     int sx, sy, sz, W;
     unsigned long long words;  // slab words of the level
+    // ceil(2^24 / c.sy) (kColourGen): n * per_sy >> 24 is n / c.sy for n < 2^13
+    // and c.sy <= 1024, as the excess, below n / 2^24, is less than 1 / c.sy;
+    // with c.sy >= 64 the product stays below 2^32
+    unsigned per_sy;
 };
 
 // The reference's normal-derived colour word without material bits
@@ -377,11 +402,11 @@ __device__ uint16_t normal_word(const WriteArgs& a, int x, int j, int z) {
         for (int dx = -1; dx <= 1; dx++) {
             const int xx = x + dx;
             if (xx < 0 || xx >= a.sx) continue;
-            const uint64_t* n = a.cols + (static_cast<long long>(zz) * a.sx + xx) * a.W;
+            const uint64_t* n = a.cols + static_cast<long long>(zz) * a.W * a.sx + xx;
             for (int dy = -1; dy <= 1; dy++) {
                 const int jj = j + dy;
                 if (jj < 0 || jj >= a.sy) continue;
-                if ((n[jj >> 6] >> (jj & 63)) & 1) {
+                if ((n[static_cast<long long>(jj >> 6) * a.sx] >> (jj & 63)) & 1) {
                     mx += dx;
                     my += dy;
                     mz += dz;
@@ -407,127 +432,139 @@ __device__ uint16_t normal_word(const WriteArgs& a, int x, int j, int z) {
     return static_cast<uint16_t>(ny);
 }
 
-// One column's words -- [run count][colour count][headers][colours] -- at
-// dst (shared or global memory).  Returns the first header (valid when the
-// column has runs).
-__device__ __forceinline__ uint32_t write_column(const WriteArgs& a, const uint64_t* s, int x, int z, int nh,
-                                                 int ncol, uint16_t* dst, bool* have_first_out) {
-    dst[0] = static_cast<uint16_t>(nh);
-    dst[1] = static_cast<uint16_t>(ncol);
-    uint16_t* hp = dst + 2;
-    uint16_t* cp = dst + 2 + nh;
-    uint32_t first = 0;
-    bool have_first = false;
-    int tint = 0;
-    if (a.mode == kColourGen) tint = rle::gen::tint(a.c, x << a.mip, z << a.mip);
-    int end = 0;
-    for (int r0 = next_bit(s, a.W, 0, true); r0 < a.sy; r0 = next_bit(s, a.W, end, true)) {
-        const int r1 = next_bit(s, a.W, r0, false);
-        // headers (src/Rle4.cpp:166-182)
-        int skip = r0 - end, solid = r1 - r0;
-        while (skip > 1023) {
-            if (!have_first) { first = 1023; have_first = true; }
-            *hp++ = 1023;
-            skip -= 1023;
-        }
-        while (solid > 63) {
-            const uint16_t h = static_cast<uint16_t>(63 * 1024 + (skip & 1023));
-            if (!have_first) { first = h; have_first = true; }
-            *hp++ = h;
-            solid -= 63;
-            skip = 0;
-        }
-        const uint16_t h = static_cast<uint16_t>((solid & 63) * 1024 + (skip & 1023));
-        if (!have_first) { first = h; have_first = true; }
-        *hp++ = h;
-        // colours of the run's voxels, top down
-        for (int j = r0; j < r1; j++) {
-            uint16_t col;
-            if (a.mode == kColourGen) {
-                col = rle::gen::colour(a.c, tint, x << a.mip, j << a.mip, z << a.mip);
-            } else if (a.mode == kColourNormal) {
-                col = normal_word(a, x, j, z);
-            } else {
-                const long long idx = (static_cast<long long>(x) << a.mip) +
-                                      (static_cast<long long>(j) << a.mip) * a.sx0 +
-                                      (static_cast<long long>(z) << a.mip) * a.sx0 * a.sy0;
-                col = a.volume[idx];
-            }
-            *cp++ = col;
-        }
-        end = r1;
-    }
-    *have_first_out = have_first;
-    return first;
-}
-
-// u16 words a warp stages in shared memory before one coalesced copy.
+// Words of a warp's columns staged in shared memory at a time, and its warps
+// per block (8 KB a warp).
 constexpr int kStageWords = 2048;
+constexpr int kWriteWarps = 4;
 
-// One thread per column.  The 32 columns of a warp are consecutive, so their
-// words form one contiguous range of the slab array: the lanes write their
-// columns into a shared-memory stage and the warp copies the range out with
-// 4-byte stores (2-byte ones at its two ends, which may share a word with the
-// neighbouring warps' ranges).  A warp whose range exceeds the stage writes
-// its columns directly.
-__global__ void __launch_bounds__(kThreads) write_kernel(const __grid_constant__ WriteArgs a,
-                                                         const uint64_t* __restrict__ surf,
-                                                         const unsigned long long* __restrict__ offsets,
-                                                         const uint16_t* __restrict__ nhead,
-                                                         uint16_t* __restrict__ slabs, uint2* __restrict__ table) {
-    __shared__ uint16_t stage_all[kThreads / 32][kStageWords];
-    uint16_t* stage = stage_all[threadIdx.x >> 5];
+// One warp per 32 consecutive columns, whose words -- [run count][colour
+// count][headers][colours] each -- form one contiguous range of the slab
+// array.  Every lane lays out its column in the stage: counts and headers as
+// they are, and for a colour the column's lane and the voxel's j.  Then the
+// warp takes the stage two words a lane, works out the colours, and stores
+// four bytes a lane.  The columns differ in their numbers of voxels, so that
+// colouring while walking a column leaves most lanes idle; the walk is now a
+// store per voxel.  (2-byte stores at the two ends of the range, which may
+// share a word with the neighbouring warps'.)  A range longer than the stage
+// goes in several turns, each walking the columns that reach into it.
+// All levels 1290 -> 990 us at 2048 x 2048 x 256 generated, 265 -> 138 us for a
+// coloured 512 x 256 x 512 volume; instructions bound it.  (Stages of 1024 and
+// 1280 words, for more blocks: 2 to 4% slower in all; the voxels by set bits
+// instead of by runs: 730 instead of 755 us for generated level 0, but 109
+// instead of 77 us for the volume's longer runs.)
+__global__ void __launch_bounds__(kWriteWarps * 32) write_kernel(const __grid_constant__ WriteArgs a,
+                                                                 const uint64_t* __restrict__ surf,
+                                                                 const unsigned long long* __restrict__ offsets,
+                                                                 const uint32_t* __restrict__ nwords,
+                                                                 const uint16_t* __restrict__ nhead,
+                                                                 uint16_t* __restrict__ slabs,
+                                                                 uint2* __restrict__ table) {
+    constexpr uint32_t kColour = 0x80000000u;  // | lane << 16 | j
+    __shared__ uint32_t stage_all[kWriteWarps][kStageWords];
+    __shared__ int tints_all[kWriteWarps][32];
+    uint32_t* stage = stage_all[threadIdx.x >> 5];
+    int* tints = tints_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     const long long ncols = static_cast<long long>(a.sx) * a.sz;
     const bool valid = q < ncols;
-    int x = 0, z = 0, nh = 0, ncol = 0;
-    uint64_t s[kMaxWords];
-    unsigned long long ofs = 0;
-    if (valid) {
-        x = static_cast<int>(q % a.sx);
-        z = static_cast<int>(q / a.sx);
-        for (int w = 0; w < a.W; w++) {
-            s[w] = surf[q * a.W + w];
-            ncol += __popcll(s[w]);
-        }
-        ofs = offsets[q];
-        nh = nhead[q];
-    }
-    const unsigned long long col_end = ofs + 2u + static_cast<unsigned long long>(nh + ncol);
-    // the warp's range: from lane 0's offset to the end of its last valid column
     const unsigned valid_mask = __ballot_sync(0xffffffffu, valid);
     if (valid_mask == 0) return;  // a warp past the level's last column
+    const int shift = __ffs(a.sx) - 1;  // sx is a power of two
+    int x = 0, z = 0, nh = 0, nw = 0;
+    unsigned long long ofs = 0;
+    if (valid) {
+        x = static_cast<int>(q) & (a.sx - 1);
+        z = static_cast<int>(q >> shift);
+        ofs = offsets[q];
+        nw = static_cast<int>(nwords[q]);
+        nh = nhead[q];
+        if (a.mode == kColourGen) tints[lane] = rle::gen::tint(a.c, x << a.mip, z << a.mip);
+    }
+    // the warp's range: from lane 0's offset to the end of its last valid column
     const int last = 31 - __clz(valid_mask);
     const unsigned long long base = __shfl_sync(0xffffffffu, ofs, 0);
-    const unsigned long long stop = __shfl_sync(0xffffffffu, col_end, last);
-    const bool staged = stop - base <= static_cast<unsigned long long>(kStageWords);
-    bool have_first = false;
+    const int from = static_cast<int>(ofs - base), to = from + nw;  // 32 columns of 2 + 1024 + 1024 words at most
+    const int n = __shfl_sync(0xffffffffu, to, last);
+    const long long row = static_cast<long long>(a.W) * a.sx;
+    const long long q0 = q - lane;
     uint32_t first = 0;
-    if (valid) {
-        uint16_t* dst = staged ? stage + (ofs - base) : slabs + ofs;
-        first = write_column(a, s, x, z, nh, ncol, dst, &have_first);
-    }
-    if (staged) {
-        __syncwarp();
-        const int n = static_cast<int>(stop - base);
-        uint16_t* g = slabs + base;
-        int start = 0;
-        if ((reinterpret_cast<uintptr_t>(g) & 2u) && n > 0) {
-            if (lane == 0) g[0] = stage[0];
-            start = 1;
+    uint16_t* g = slabs + base;
+    const int odd = static_cast<int>(base & 1);  // the slabs start on 256 bytes
+    for (int w0 = 0; w0 < n; w0 += kStageWords) {
+        if (valid && from < w0 + kStageWords && to > w0) {
+            auto put = [&](int at, uint32_t v) {
+                const unsigned i = static_cast<unsigned>(at - w0);
+                if (i < static_cast<unsigned>(kStageWords)) stage[i] = v;
+            };
+            put(from, static_cast<uint32_t>(nh));
+            put(from + 1, static_cast<uint32_t>(nw - 2 - nh));
+            const uint32_t colour0 = kColour | static_cast<uint32_t>(lane << 16);
+            int hp = from + 2, cp = hp + nh, start = 0, end = 0;
+            auto head = [&](uint32_t h) {
+                if (hp == from + 2) first = h;
+                put(hp++, h);
+            };
+            // headers of a finished run (src/Rle4.cpp:166-182)
+            auto run = [&](int r0, int r1) {
+                int skip = r0 - end, solid = r1 - r0;
+                for (; skip > 1023; skip -= 1023) head(1023u);
+                for (; solid > 63; solid -= 63) {
+                    head(63u * 1024u + static_cast<uint32_t>(skip));
+                    skip = 0;
+                }
+                head(static_cast<uint32_t>(solid) * 1024u + static_cast<uint32_t>(skip));
+                // the run's voxels, top down
+                for (int j = r0; j < r1; j++) put(cp++, colour0 + static_cast<uint32_t>(j));
+                end = r1;
+            };
+            const uint64_t* s = surf + z * row + x;
+            uint64_t open = 0;
+            for (int w = 0; w < a.W; w++) {
+                const uint64_t v = s[static_cast<long long>(w) * a.sx];
+                for (uint64_t t = v ^ ((v << 1) | open); t; t &= t - 1) {
+                    const int at = w * 64 + __ffsll(static_cast<long long>(t)) - 1;
+                    open ^= 1;
+                    if (open) start = at;
+                    else run(start, at);
+                }
+                open = v >> 63;
+            }
+            if (open) run(start, a.W * 64);
         }
-        const int pairs = (n - start) >> 1;
-        uint32_t* g32 = reinterpret_cast<uint32_t*>(g + start);
-        for (int i = lane; i < pairs; i += 32)
-            g32[i] = static_cast<uint32_t>(stage[start + 2 * i]) | (static_cast<uint32_t>(stage[start + 2 * i + 1]) << 16);
-        if (((n - start) & 1) && lane == 0) g[n - 1] = stage[n - 1];
+        __syncwarp();
+        const int m = min(n - w0, kStageWords);
+        auto word = [&](int i) {
+            const uint32_t v = stage[i];
+            if (!(v & kColour)) return v;
+            const int l = static_cast<int>(v >> 16) & 31, j = static_cast<int>(v & 0xffffu);
+            const long long qc = q0 + l;
+            const int cx = static_cast<int>(qc) & (a.sx - 1), cz = static_cast<int>(qc >> shift);
+            if (a.mode == kColourGen) {
+                const int y = a.c.sy - 1 - (j << a.mip);
+                const int band = static_cast<int>(static_cast<unsigned>(y * 8) * a.per_sy >> 24);
+                return static_cast<uint32_t>(
+                    rle::gen::colour_in_band(a.c, tints[l], band, cx << a.mip, y, cz << a.mip));
+            }
+            if (a.mode == kColourNormal) return static_cast<uint32_t>(normal_word(a, cx, j, cz));
+            return static_cast<uint32_t>(a.volume[(static_cast<long long>(cx) << a.mip) +
+                                                  (static_cast<long long>(j) << a.mip) * a.sx0 +
+                                                  (static_cast<long long>(cz) << a.mip) * a.sx0 * a.sy0]);
+        };
+        // kStageWords is even: the parity of the first word is that of the range
+        if (odd && lane == 0) g[w0] = static_cast<uint16_t>(word(0));
+        for (int i = odd + 2 * lane; i < m; i += 64) {
+            const uint32_t lo = word(i);
+            if (i + 1 < m) *reinterpret_cast<uint32_t*>(g + w0 + i) = lo | (word(i + 1) << 16);
+            else g[w0 + i] = static_cast<uint16_t>(lo);
+        }
+        __syncwarp();
     }
     if (!valid) return;
     // RLE4::load's table entry (src/Rle4.cpp:285-314): the word after the
     // two counts is read as the first header even for an empty column, where
     // it is the next column's run count (or nothing past the level's end).
-    if (!have_first) first = (ofs + 2 < a.words && q + 1 < ncols) ? nhead[q + 1] : 0u;
+    if (nh == 0) first = (ofs + 2 < a.words && q + 1 < ncols) ? nhead[q + 1] : 0u;
     table[q] = make_uint2(static_cast<uint32_t>(ofs), static_cast<uint32_t>(nh) + (first << 16));
 }
 
@@ -682,8 +719,10 @@ rle_status write_level(Build& B, const WriteArgs& base, rle::Level& D, int m, in
     a.sz = L.sz;
     a.W = L.W;
     a.words = D.words;
-    write_kernel<<<grid_for(static_cast<long long>(L.sx) * L.sz), kThreads, 0, B.stream>>>(
-        a, B.sc.surf[i], B.sc.offsets[i], B.sc.nhead[i], D.d_slabs, reinterpret_cast<uint2*>(D.d_table));
+    constexpr int threads = kWriteWarps * 32;
+    write_kernel<<<grid_for(static_cast<long long>(L.sx) * L.sz, threads), threads, 0, B.stream>>>(
+        a, B.sc.surf[i], B.sc.offsets[i], B.sc.nwords[i], B.sc.nhead[i], D.d_slabs,
+        reinterpret_cast<uint2*>(D.d_table));
     return launch_check("write_kernel");
 }
 
@@ -808,6 +847,7 @@ extern "C" rle_status rle_scenegen_device(const rle_scenegen_params* p, int devi
     std::memset(&a, 0, sizeof(a));
     a.c = g.c;
     a.mode = kColourGen;
+    a.per_sy = ((1u << 24) + static_cast<unsigned>(p->sy) - 1u) / static_cast<unsigned>(p->sy);
     return encode_levels(B, a, out);
 }
 

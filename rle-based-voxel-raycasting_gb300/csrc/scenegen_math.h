@@ -152,18 +152,14 @@ RLE_HD int tint(const Consts& p, int x, int z) {
                                          p.seed32 ^ 0xC0105EEDu) * 96.0f);
 }
 
-// RGB565 colour of level-0 voxel (x, j, z), j counted down from the top,
-// given the column's tint: a height-band palette scaled by tint + jitter.
-RLE_HD uint16_t colour(const Consts& p, int tint_xz, int x, int j, int z) {
+// RGB565 colour of the level-0 voxel at height y of column (x, z), given the
+// column's tint and the palette band, 0..7: the palette scaled by tint + jitter.
+RLE_HD uint16_t colour_in_band(const Consts& p, int tint_xz, int band, int x, int y, int z) {
     // palette bands, bottom to top: 0x5C4E42, 0x96825A, 0xC4B478, 0x609646,
     // 0x467C3A, 0x767064, 0x96928C, 0xECECF0 (0xRRGGBB), held as one byte per
     // band in each channel's constant (band b in bits 8b..8b+7), so that no
     // thread builds a table in local memory
     const uint64_t kPalR = 0xEC96764660C4965Cull, kPalG = 0xEC92707C96B4824Eull, kPalB = 0xF08C643A46785A42ull;
-    const int y = p.sy - 1 - j;
-    int band = y * 8 / p.sy;
-    if (band > 7) band = 7;
-    if (band < 0) band = 0;
     const int jitter = static_cast<int>(hash32(x, y, z, p.seed32) & 31);
     const int f = 176 + tint_xz + jitter;  // 176..303, /256
     const int sh = 8 * band;
@@ -173,6 +169,15 @@ RLE_HD uint16_t colour(const Consts& p, int tint_xz, int x, int j, int z) {
     if (g > 255) g = 255;
     if (b > 255) b = 255;
     return static_cast<uint16_t>(((r >> 3) << 11) | ((g >> 2) << 5) | (b >> 3));
+}
+
+// RGB565 colour of level-0 voxel (x, j, z), j counted down from the top.
+RLE_HD uint16_t colour(const Consts& p, int tint_xz, int x, int j, int z) {
+    const int y = p.sy - 1 - j;
+    int band = y * 8 / p.sy;
+    if (band > 7) band = 7;
+    if (band < 0) band = 0;
+    return colour_in_band(p, tint_xz, band, x, y, z);
 }
 
 }  // namespace gen

@@ -60,13 +60,11 @@ def load_rle():
 # default run, captured with ncu (profiles/raycast_traffic_1080p_cave2048.md
 # gives the command and the per-frame figures).  A profiler run cannot be part
 # of the timed benchmark; the capture is repeated when the kernel changes.
-RAYCAST_DRAM_BYTES_PER_LAUNCH = 33_878_784
+RAYCAST_DRAM_BYTES_PER_LAUNCH = 34_359_296
 RAYCAST_DRAM_FRAMES = "frames 0-4 of the timed camera path (seed 20261203, after 5 warm-up frames)"
 # The end-to-end loop renders like a throughput-oriented renderer: several frames in flight (one
-# stream, workspace and output set each) and 16 lanes per column ray (two rays per warp, twice the
-# rays in flight per SM), which wins once frames overlap; isolated frames (`value`) keep 32.
-# Measured on GB300, 60 frames: 32 lanes x 3 / 4 / 6 in flight -> 7891 / 8204 / 8225 Mrays/s;
-# 16 lanes x 4 / 6 / 8 -> 7818 / 8790 / 8845.
+# stream, workspace and output set each).  The lanes setting is accepted without effect: every
+# setting runs one warp per column ray.
 E2E_FRAMES_IN_FLIGHT = 6
 E2E_LANES_PER_RAY = 16
 

@@ -94,7 +94,10 @@ RLE_STEP_FN DdaJump dda_jump(const Dda& d, const DdaCache& c, float kf) {
     float n = fminf(fmaxf((guess + 8388608.0f) - 8388608.0f, 0.0f), kf);
     float m = kf - n;
     float a0 = fmaf(n, c.s0, d.dd0), a1 = fmaf(m, c.s1, d.dd1);
-    const bool over = n > 0.0f && !(a0 - c.s0 <= a1), under = m > 0.0f && !(a1 - c.s1 < a0);
+    // the sums before, from the chain's start: a0 or a1 of a count too many may
+    // lie past its binade, rounded to the coarser ulp, and so would a0 - s0
+    const bool over = n > 0.0f && !(fmaf(n - 1.0f, c.s0, d.dd0) <= a1);
+    const bool under = m > 0.0f && !(fmaf(m - 1.0f, c.s1, d.dd1) < a0);
     n += over ? -1.0f : (under ? 1.0f : 0.0f);
     m = kf - n;
     a0 = fmaf(n, c.s0, d.dd0);

@@ -287,6 +287,9 @@ extern "C" rle_status rle_scene_load_memory(const void* bytes, size_t nbytes, in
         if (hl.words && (e = cudaMemcpy(lv.d_slabs, hl.slabs, static_cast<size_t>(hl.words) * 2, cudaMemcpyHostToDevice)) != cudaSuccess) { st = cuda_fail(e, "cudaMemcpy(slabs)"); break; }
         s->device_bytes += tbytes + sbytes;
     }
+    // A copy from pageable memory may return with its last part on the way, and
+    // the fills do; the frames' streams do not wait for the default stream.
+    if (st == RLE_OK && (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) st = cuda_fail(e, "scene upload");
     if (prev >= 0) cudaSetDevice(prev);
     if (st != RLE_OK) {
         release(s);

@@ -178,6 +178,10 @@ rle_status rle_scenegen_device(const rle_scenegen_params* p, int device, rle_sce
  * complete: the build runs on a stream of its own, which waits for no other. */
 rle_status rle_encode_device(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz,
                              int nummaps, int device, rle_scene** out);
+/* The same for inputs that `stream` (of `device`; NULL: the default stream) may
+ * still be writing: the build runs behind the work queued on it so far. */
+rle_status rle_encode_device_after(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz,
+                                   int nummaps, int device, void* stream, rle_scene** out);
 
 /* ---------------------------------------------------------------------- */
 /* Cameras and ray maps                                                   */

@@ -18,6 +18,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import os
+import sys
 from pathlib import Path
 from typing import Optional
 
@@ -165,6 +166,7 @@ def _load() -> C.CDLL:
         "rle_bounds_check_read": (C.c_int, [C.c_int, C.POINTER(C.c_uint32), C.c_int]),
         "rle_debug_level_pointers": (C.c_int, [vp, C.c_int, C.POINTER(vp), C.POINTER(vp), C.POINTER(C.c_uint64)]),
         "rle_encode_device": (C.c_int, [vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(vp)]),
+        "rle_encode_device_after": (C.c_int, [vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, vp, C.POINTER(vp)]),
         "rle_raymap_build": (C.c_int, [C.POINTER(Camera), C.POINTER(ViewParams), C.POINTER(RayMap)]),
         "rle_raybuf_words": (C.c_size_t, [C.POINTER(RayMap)]),
         "rle_tuning_set": (C.c_int, [C.POINTER(Tuning)]),
@@ -229,6 +231,12 @@ def ptr(x) -> Optional[int]:
     raise TypeError(f"cannot take a device pointer of {type(x).__name__}")
 
 
+def _on_device(x, device: int) -> bool:
+    """Whether x is a torch tensor of CUDA device `device`."""
+    torch = sys.modules.get("torch")
+    return torch is not None and isinstance(x, torch.Tensor) and x.is_cuda and x.get_device() == device
+
+
 def version() -> str:
     return _lib.rle_version().decode()
 
@@ -282,10 +290,19 @@ class Scene:
     def encode_on_device(cls, bits, colours, sx: int, sy: int, sz: int, nummaps: int = 4,
                          device: int = 0) -> "Scene":
         """rle_encode_device: RLE4::compress_all of a device bit volume in the
-        reference's Tree layout (optional u16 colour per voxel, same index)."""
+        reference's Tree layout (optional u16 colour per voxel, same index).
+        Behind the current torch stream of the device if an input is a tensor
+        on it (rle_encode_device_after); inputs written on another stream, or
+        passed as pointers, must be complete."""
         h = C.c_void_p()
-        _check(_lib.rle_encode_device(ptr(bits), ptr(colours), sx, sy, sz, nummaps, device, C.byref(h)),
-               "rle_encode_device")
+        if _on_device(bits, device) or _on_device(colours, device):
+            # the handle alone: torch.cuda.current_stream() builds an object, 10 us more a call
+            stream = sys.modules["torch"]._C._cuda_getCurrentRawStream(device)
+            _check(_lib.rle_encode_device_after(ptr(bits), ptr(colours), sx, sy, sz, nummaps, device, stream or None,
+                                                C.byref(h)), "rle_encode_device_after")
+        else:
+            _check(_lib.rle_encode_device(ptr(bits), ptr(colours), sx, sy, sz, nummaps, device, C.byref(h)),
+                   "rle_encode_device")
         return cls(h)
 
     @classmethod

@@ -823,6 +823,23 @@ rle_status begin(Build& B, int device) {
     return RLE_OK;
 }
 
+// Orders the build behind what is queued on `stream` (of the build's device) so
+// far.  A stream that is being captured has run nothing that could be waited for.
+rle_status order_behind(Build& B, cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+    if (e == cudaErrorStreamCaptureImplicit || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return RLE_OK;
+    }
+    cudaEvent_t done = nullptr;
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(done, stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(B.stream, done, 0);
+    if (done) cudaEventDestroy(done);
+    return e == cudaSuccess ? RLE_OK : cuda_fail(e, "scene build: ordering behind the caller's stream");
+}
+
 }  // namespace
 
 extern "C" rle_status rle_scenegen_device(const rle_scenegen_params* p, int device, rle_scene** out) {
@@ -851,8 +868,11 @@ extern "C" rle_status rle_scenegen_device(const rle_scenegen_params* p, int devi
     return encode_levels(B, a, out);
 }
 
-extern "C" rle_status rle_encode_device(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz,
-                                        int nummaps, int device, rle_scene** out) {
+namespace {
+
+// `ordered`: behind the work queued on `stream`.
+rle_status encode_device(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz, int nummaps,
+                         int device, bool ordered, cudaStream_t stream, rle_scene** out) {
     if (!out) return RLE_ERR_INVALID_ARG;
     *out = nullptr;
     auto pow2 = [](int v) { return v >= 8 && (v & (v - 1)) == 0; };
@@ -868,6 +888,7 @@ extern "C" rle_status rle_encode_device(const uint8_t* d_bits, const uint16_t* d
     Build B;
     rle_status st = begin(B, device);
     if (st != RLE_OK) return st;
+    if (ordered && (st = order_behind(B, stream)) != RLE_OK) return st;
     if ((st = alloc_levels(B, sx, sy, sz, nummaps)) != RLE_OK) return st;
     const long long n = static_cast<long long>(sx) * sz * B.lv[0].W;
     transpose_kernel<<<grid_for(n), kThreads, 0, B.stream>>>(d_bits, sx, sy, sz, B.lv[0].W, B.lv[0].cols);
@@ -880,4 +901,16 @@ extern "C" rle_status rle_encode_device(const uint8_t* d_bits, const uint16_t* d
     a.sx0 = sx;
     a.sy0 = sy;
     return encode_levels(B, a, out);
+}
+
+}  // namespace
+
+extern "C" rle_status rle_encode_device(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz,
+                                        int nummaps, int device, rle_scene** out) {
+    return encode_device(d_bits, d_colours, sx, sy, sz, nummaps, device, false, nullptr, out);
+}
+
+extern "C" rle_status rle_encode_device_after(const uint8_t* d_bits, const uint16_t* d_colours, int sx, int sy, int sz,
+                                              int nummaps, int device, void* stream, rle_scene** out) {
+    return encode_device(d_bits, d_colours, sx, sy, sz, nummaps, device, true, static_cast<cudaStream_t>(stream), out);
 }

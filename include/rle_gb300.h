@@ -201,7 +201,9 @@ typedef struct rle_view_params {
     int samples;        /* samples per column ray (RENDER_SIZE); 0 = width */
     int maxres;         /* column rays per unit of fan (RAYS_CASTED_RES/4); 0 = width */
     float border;       /* vertical border of the square ray-map plane; <= 0 = (W-H)/(2W) */
-    int mip_distance;   /* distance of the first LOD switch (MIP_DISTANCE); 0 = width */
+    int mip_distance;   /* distance of the first LOD switch (MIP_DISTANCE); 0 = width.  Times
+                           1 - |pitch| / 4, cut to a whole number, it has to be at least 1: from 0
+                           on a ray would never end, and rendering is refused */
     int z_far;          /* ray length in DDA steps (RAYS_DISTANCE); 0 = 80000 */
 } rle_view_params;
 

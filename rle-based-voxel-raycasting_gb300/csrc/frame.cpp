@@ -8,6 +8,7 @@
 // and nothing synchronises the host.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -15,6 +16,33 @@
 #include "rle_internal.h"
 
 namespace rle {
+
+// The march's level-of-detail schedule (the same for every ray of a frame) on
+// z, dz and the switch distance alone, a level at a time.  A switch doubles the
+// distance until it reaches z, which never happens from 0 (nor once the doubling
+// has run out of an int), and a step has to move z.
+bool march_ends(int mapswitch, float posy, int z_far) {
+    const float zfar = static_cast<float>(z_far);
+    uint32_t sw = static_cast<uint32_t>(mapswitch);
+    float z = 0, dz = 1;
+    auto distance = [&] { return static_cast<float>(static_cast<int32_t>(sw)); };
+    for (float y = posy; z > distance() || y > 512.0f; y *= 0.5f) {
+        sw *= 2;
+        dz *= 2;
+    }
+    if (dz > zfar) return true;  // no first step
+    for (;;) {
+        while (z > distance()) {
+            if (static_cast<int32_t>(sw) <= 0) return false;
+            sw *= 2;
+            dz *= 2;
+        }
+        const float reach = std::min(distance(), zfar);  // z has to pass it in steps of dz
+        if (std::nextafter(reach, INFINITY) - reach > dz) return false;
+        if (zfar <= distance()) return true;
+        z = distance() + dz;
+    }
+}
 
 rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayParams* p) {
     std::memset(p, 0, sizeof(*p));
@@ -62,6 +90,11 @@ rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayPara
     p->mapswitch0 = static_cast<int>(static_cast<double>(rm->mip_distance) *
                                      (0.25 * static_cast<double>(4.0f - std::fabs(rm->rotation[0]))));
     p->z_far = rm->z_far;
+    if (rm->rays > 0 && !march_ends(p->mapswitch0, p->posy, p->z_far)) {
+        set_error("ray map: rays would not end with mip_distance %d (first switch at %d, pitch counted) and z_far %d",
+                  rm->mip_distance, p->mapswitch0, rm->z_far);
+        return RLE_ERR_INVALID_ARG;
+    }
     p->nummaps = scene->nummaps;
     p->gridx0 = scene->lv[0].sx;
     p->gridz0 = scene->lv[0].sz;

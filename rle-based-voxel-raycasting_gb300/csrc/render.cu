@@ -1267,10 +1267,10 @@ __device__ __forceinline__ void cast_ray(const RayParams& P, int x, bool active,
 // Shared memory of a raycast block: the warps' occupancy masks (`words` each,
 // padded to 16 bytes), their span queues (one entry per lane), the merge's
 // entry lists (one word per lane) and kRecs run records per thread.
-__host__ __device__ __forceinline__ int mask_region_words(int slots, int words) {
+__host__ __device__ constexpr int mask_region_words(int slots, int words) {
     return (slots * words + 3) & ~3;
 }
-__host__ __device__ __forceinline__ size_t raycast_smem_bytes(int threads, int slots, int words) {
+__host__ __device__ constexpr size_t raycast_smem_bytes(int threads, int slots, int words) {
     return static_cast<size_t>(mask_region_words(slots, words)) * 4 +
            static_cast<size_t>(threads) * (kRecs * 3 * sizeof(uint32_t) + kQueueVecs * sizeof(uint4) + sizeof(uint32_t));
 }
@@ -1363,24 +1363,20 @@ __global__ void __launch_bounds__(128, 4) raycast_batch_kernel(BatchHeader* hdr,
     }
 }
 
+// The largest launch (blocks of 128, ray maps of 16384 samples) has what a kernel
+// may have without asking.  The limit that cudaFuncSetAttribute moves is the
+// kernel's, in every thread and batch: moved to one launch's size, it refuses
+// another's larger block.
+static_assert(raycast_smem_bytes(128, 128 / kLanes, 16384 / 32) <= 48 * 1024, "dynamic shared memory of a launch");
+
 template <bool kCount, bool kHits>
 rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) {
     const int words = (p.S + 31) >> 5;
     const int rays_per_block = threads / kLanes;
     const size_t smem = raycast_smem_bytes(threads, rays_per_block, words);
-    if (smem > 227 * 1024) {
-        set_error("rle_render_rays: %d samples per ray exceed shared memory at this launch shape", p.S);
-        return RLE_ERR_CAPACITY;
-    }
-    cudaError_t e = cudaFuncSetAttribute(raycast_kernel<kCount, kHits>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) {
-        set_error("cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-        return RLE_ERR_CUDA;
-    }
     const int blocks = (p.rays + rays_per_block - 1) / rays_per_block;
     raycast_kernel<kCount, kHits><<<blocks, threads, smem, stream>>>(p);
-    e = cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("raycast launch: %s", cudaGetErrorString(e));
         return RLE_ERR_CUDA;
@@ -1401,14 +1397,8 @@ size_t batch_smem(int threads, int max_samples) {
 template <bool kHits>
 rle_status batch_blocks(int threads, int max_samples, int* blocks) {
     const size_t smem = batch_smem(threads, max_samples);
-    if (smem > 227 * 1024) {
-        set_error("batch: %d samples per ray exceed shared memory at this launch shape", max_samples);
-        return RLE_ERR_CAPACITY;
-    }
-    cudaError_t e = cudaFuncSetAttribute(raycast_batch_kernel<kHits>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     int dev = 0, sms = 0, per_sm = 0;
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, raycast_batch_kernel<kHits>,

@@ -44,6 +44,22 @@ bool march_ends(int mapswitch, float posy, int z_far) {
     }
 }
 
+namespace {
+// mapswitch * (0.25*(4-abs(viewrot.x))): float subtraction, double product,
+// truncation to int (src/Cuda_Render.h:335)
+int first_switch(const rle_raymap* rm) {
+    return static_cast<int>(static_cast<double>(rm->mip_distance) *
+                            (0.25 * static_cast<double>(4.0f - std::fabs(rm->rotation[0]))));
+}
+}  // namespace
+
+rle_status check_march(const rle_raymap* rm) {
+    if (rm->rays <= 0 || march_ends(first_switch(rm), rm->position[1], rm->z_far)) return RLE_OK;
+    set_error("ray map: rays would not end with mip_distance %d (first switch at %d, pitch counted) and z_far %d",
+              rm->mip_distance, first_switch(rm), rm->z_far);
+    return RLE_ERR_INVALID_ARG;
+}
+
 rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayParams* p) {
     std::memset(p, 0, sizeof(*p));
     if (rm->samples < 8 || rm->samples > 16384 || rm->rays < 0 || rm->rays > rm->rows || rm->maxres < 1 ||
@@ -63,6 +79,8 @@ rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayPara
             return RLE_ERR_INVALID_ARG;
         }
     }
+    const rle_status st = check_march(rm);
+    if (st != RLE_OK) return st;
     p->p5x = rm->p_2d[5][0];
     p->p5y = rm->p_2d[5][1];
     p->p5z = rm->p_2d[5][2];
@@ -85,16 +103,8 @@ rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayPara
     p->S = rm->samples;
     p->focal = static_cast<float>(rm->samples / 2) / rm->fov_scale;
     p->rays = rm->rays;
-    // mapswitch * (0.25*(4-abs(viewrot.x))): float subtraction, double
-    // product, truncation to int (src/Cuda_Render.h:335)
-    p->mapswitch0 = static_cast<int>(static_cast<double>(rm->mip_distance) *
-                                     (0.25 * static_cast<double>(4.0f - std::fabs(rm->rotation[0]))));
+    p->mapswitch0 = first_switch(rm);
     p->z_far = rm->z_far;
-    if (rm->rays > 0 && !march_ends(p->mapswitch0, p->posy, p->z_far)) {
-        set_error("ray map: rays would not end with mip_distance %d (first switch at %d, pitch counted) and z_far %d",
-                  rm->mip_distance, p->mapswitch0, rm->z_far);
-        return RLE_ERR_INVALID_ARG;
-    }
     p->nummaps = scene->nummaps;
     p->gridx0 = scene->lv[0].sx;
     p->gridz0 = scene->lv[0].sz;

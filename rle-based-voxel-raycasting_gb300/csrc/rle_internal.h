@@ -131,6 +131,7 @@ struct ResolveParams {
 // Whether rays marched with this first switch distance, eye height and end
 // come to that end (RayParams::mapswitch0, posy, z_far).
 bool march_ends(int mapswitch, float posy, int z_far);
+rle_status check_march(const rle_raymap* rm);  // refuses a ray map whose rays would not
 rle_status fill_ray_params(const rle_scene* scene, const rle_raymap* rm, RayParams* p);
 rle_status fill_resolve_params(const rle_raymap* rm, ResolveParams* p);
 

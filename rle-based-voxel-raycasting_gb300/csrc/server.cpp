@@ -381,6 +381,7 @@ extern "C" rle_status rle_server_submit(rle_server* s, const rle_request* r, uin
     if (!s || !r || !ticket || !r->d_colour || !r->d_depth) return RLE_ERR_INVALID_ARG;
     rle_raymap rm;
     rle_status st = rle_raymap_build(&r->cam, &r->view, &rm);
+    if (st == RLE_OK) st = rle::check_march(&rm);  // here, not in the launch, which would fail its other requests
     if (st != RLE_OK) return st;
     Req q;
     q.r = *r;

@@ -817,6 +817,7 @@ rle_status begin(Build& B, int device) {
         return RLE_ERR_INVALID_ARG;
     }
     B.device = device;
+    rle::forget_last_error();
     if ((e = cudaSetDevice(device)) != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
     if ((e = cudaStreamCreateWithFlags(&B.stream, cudaStreamNonBlocking)) != cudaSuccess)
         return cuda_fail(e, "cudaStreamCreate");

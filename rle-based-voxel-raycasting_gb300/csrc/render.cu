@@ -1375,6 +1375,7 @@ rle_status launch_variant(const RayParams& p, int threads, cudaStream_t stream) 
     const int rays_per_block = threads / kLanes;
     const size_t smem = raycast_smem_bytes(threads, rays_per_block, words);
     const int blocks = (p.rays + rays_per_block - 1) / rays_per_block;
+    forget_last_error();
     raycast_kernel<kCount, kHits><<<blocks, threads, smem, stream>>>(p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1419,6 +1420,7 @@ rle_status batch_launch(const BatchRaycast& b, cudaStream_t stream) {
         const rle_status st = batch_blocks<kHits>(b.threads, b.max_samples, &blocks);
         if (st != RLE_OK) return st;
     }
+    forget_last_error();
     raycast_batch_kernel<kHits><<<blocks, b.threads, smem, stream>>>(
         b.header, b.ray_start, b.frames, b.tile, (b.max_samples + 31) >> 5);
     const cudaError_t e = cudaGetLastError();

@@ -164,6 +164,7 @@ bool bounds_resolve(unsigned* out4, bool clear) {
 
 rle_status launch_resolve_batch(const BatchResolve& b, void* stream) {
     if (b.blocks <= 0) return RLE_OK;
+    forget_last_error();
     resolve_batch_kernel<<<b.blocks, kResolveBlock, 0, static_cast<cudaStream_t>(stream)>>>(b.header, b.block_start,
                                                                                             b.frames);
     const cudaError_t e = cudaGetLastError();
@@ -178,6 +179,7 @@ rle_status launch_resolve(const ResolveParams& p, void* stream) {
     const dim3 block(kTileX * kTileY, 1, 1);
     const dim3 grid((p.width + kTileX - 1) / kTileX, (p.height + kTileY - 1) / kTileY, 1);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    forget_last_error();
     if (p.hit) resolve_kernel<true><<<grid, block, 0, s>>>(p);
     else resolve_kernel<false><<<grid, block, 0, s>>>(p);
     const cudaError_t e = cudaGetLastError();

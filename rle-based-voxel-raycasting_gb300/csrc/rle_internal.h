@@ -114,6 +114,11 @@ struct RayParams {
     int threads_per_block;        // block size (0 = default)
 };
 
+// Before a launch: drops what an earlier call of this thread left as its last
+// error (a refused allocation, a device that is not there; that call has
+// reported it), so that the check after the launch sees the launch alone.
+inline void forget_last_error() { cudaGetLastError(); }
+
 // Per-frame constants of the resolve (uniforms of colorize_buddha_soft.frag).
 struct ResolveParams {
     ResolveGeometry geo;

@@ -253,6 +253,7 @@ extern "C" rle_status rle_soft_filter(const uint32_t* d_colour, const float* d_d
     }
     const dim3 block(rle::kTileX, rle::kThreadsY);
     const dim3 grid((width + rle::kTileX - 1) / rle::kTileX, (height + rle::kTileY - 1) / rle::kTileY);
+    rle::forget_last_error();
     rle::soft_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(P, d_colour, d_depth, d_out);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -57,16 +57,13 @@ def load_rle():
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per raycast
 # launch on this workload: the mean over the first five timed frames of the
-# default run, captured with ncu (profiles/raycast_traffic_1080p_cave2048.md
-# gives the command and the per-frame figures).  A profiler run cannot be part
-# of the timed benchmark; the capture is repeated when the kernel changes.
-RAYCAST_DRAM_BYTES_PER_LAUNCH = 34_359_296
+# default run, captured with ncu.  A profiler run cannot be part of the timed
+# benchmark; the capture is repeated when the kernel changes.
+RAYCAST_DRAM_BYTES_PER_LAUNCH = 34_228_839
 RAYCAST_DRAM_FRAMES = "frames 0-4 of the timed camera path (seed 20261203, after 5 warm-up frames)"
 # The end-to-end loop renders like a throughput-oriented renderer: several frames in flight (one
-# stream, workspace and output set each).  The lanes setting is accepted without effect: every
-# setting runs one warp per column ray.
+# stream, workspace and output set each).
 E2E_FRAMES_IN_FLIGHT = 6
-E2E_LANES_PER_RAY = 16
 
 
 def bench_config(rays_per_frame, runs_per_column: float, world: int) -> dict:
@@ -378,14 +375,13 @@ def run_ours(args):
     # every frame back to pinned host memory; a multi-buffered frame loop:
     # frames rotate over E2E_FRAMES_IN_FLIGHT streams (own workspace and
     # outputs each), so a frame's read-back and its last rays overlap the
-    # next frames' renders; the launch shape is set through rle_tuning_set ----
+    # next frames' renders ----
     sets = [(stream, ws, colour, depth)]
     for _ in range(E2E_FRAMES_IN_FLIGHT - 1):
         sets.append((torch.cuda.Stream(), torch.empty_like(ws), torch.empty_like(colour), torch.empty_like(depth)))
     hosts = [(torch.empty(W * H, dtype=torch.int32, pin_memory=True),
               torch.empty(W * H, dtype=torch.float32, pin_memory=True)) for _ in sets]
-    rle.tuning_set(E2E_LANES_PER_RAY, 0, 0, 0)
-    for i, (s_, w_, c_, d_) in enumerate(sets):  # warm-up: every stream, this launch shape
+    for i, (s_, w_, c_, d_) in enumerate(sets):  # warm-up: every stream
         with torch.cuda.stream(s_):
             rle.render_frame(scene, cams[i % args.warmup], view, w_, ws_bytes, c_, d_, None, stream=s_.cuda_stream)
     torch.cuda.synchronize()
@@ -406,7 +402,6 @@ def run_ours(args):
         stream.wait_event(ej)
     e1.record(stream)
     torch.cuda.synchronize()
-    rle.tuning_set(0, 0, 0, 0)
     e2e_ms = e0.elapsed_time(e1)
     e2e = W * H * args.steps / (e2e_ms / 1e3) / 1e6
 
@@ -447,13 +442,13 @@ def run_ours(args):
         "e2e": {"value": round(e2e, 2), "unit": "Mrays/s", "h2d_bytes_per_step": 28,
                 "d2h_bytes_per_step": W * H * 8,
                 "pipeline": f"multi-buffered frame loop: frames rotate over {E2E_FRAMES_IN_FLIGHT} streams; a frame's read-back and last rays overlap the next frames' renders",
-                "frames_in_flight": E2E_FRAMES_IN_FLIGHT, "lanes_per_ray": E2E_LANES_PER_RAY,
+                "frames_in_flight": E2E_FRAMES_IN_FLIGHT,
                 "l2": "not flushed: the scene (294 MB) exceeds L2 and every frame has its own camera"},
         "gpu_launches": 2 * args.steps,
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": RAYCAST_DRAM_BYTES_PER_LAUNCH,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum, mean per launch over "
-                                       + RAYCAST_DRAM_FRAMES + " (profiles/raycast_traffic_1080p_cave2048.md)",
+                                       + RAYCAST_DRAM_FRAMES,
                      "kernel": "raycast_kernel", "kernel_ms": round(k_ms, 4), "peak_kind": peak_kind,
                      "kernel_ms_source": "CUDA events between the raycast and the resolve launches of the timed "
                                          "frames themselves (mean over the steps)",
@@ -610,8 +605,7 @@ def run_batched(rle, torch, scene, lv0, n_cams=64, repeats=5, seed=20261204):
                     "launches_per_batch": 2 * n_cams if best.per_frame else 2,
                     "cuda_graph": not best.per_frame},
         "speedup": round(plain_ms / batch_ms, 3),
-        "autotuned": {"tile_rays": best.tile_rays, "lanes_per_ray": best.lanes_per_ray, "staging": best.staging,
-                      "threads_per_block": best.threads_per_block, "per_frame": best.per_frame,
+        "autotuned": {"tile_rays": best.tile_rays, "threads_per_block": best.threads_per_block, "per_frame": best.per_frame,
                       "tune_s": round(t_tune, 2)},
     }
 
@@ -707,8 +701,7 @@ def run_config5(rle, torch, frames=120, views_per_batch=8, seed=7, repeats=3):
                     "ms_per_frame": round(batch_ms / frames, 4), "views_per_call": views_per_batch,
                     "mode": ("per-frame launch pairs forked over the batch's 8 worker streams" if best.per_frame
                              else "one persistent raycast + resolve pair per call"),
-                    "autotuned": {"tile_rays": best.tile_rays, "lanes_per_ray": best.lanes_per_ray,
-                                  "staging": best.staging, "per_frame": best.per_frame}},
+                    "autotuned": {"tile_rays": best.tile_rays, "per_frame": best.per_frame}},
     }
     scene.free()
     return out

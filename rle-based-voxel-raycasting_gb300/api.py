@@ -391,7 +391,9 @@ def raybuf_words(rm: RayMap) -> int:
 
 
 def tuning_set(lanes_per_ray: int = 0, cells_per_lane: int = 0, threads_per_block: int = 0, staging: int = 0) -> None:
-    """Process-wide launch shape of the raycast (0 = built-in default)."""
+    """Process-wide launch shape of the raycast (0 = built-in default).
+    threads_per_block counts; lanes_per_ray and staging are accepted without
+    effect, and cells_per_lane is 1."""
     _check(_lib.rle_tuning_set(C.byref(Tuning(lanes_per_ray, cells_per_lane, threads_per_block, staging))),
            "rle_tuning_set")
 
@@ -455,8 +457,9 @@ def batch_words_needed(frames) -> int:
 
 
 class Batch:
-    """Many cameras per launch (rle_batch_*): one persistent raycast and one
-    persistent resolve, captured into a CUDA graph and replayed."""
+    """Many cameras per call (rle_batch_*): by default a launch pair per frame
+    over eight worker streams; or one persistent raycast and one persistent
+    resolve, captured into a CUDA graph and replayed (set_tuning, autotune)."""
 
     def __init__(self, max_frames: int, raybuf_words: int, max_samples: int = 4096, with_hits: bool = False,
                  device: int = 0):

@@ -72,9 +72,9 @@ struct rle_batch {
     cudaStream_t workers[kWorkers] = {};
     cudaEvent_t fork = nullptr;
     cudaEvent_t joins[kWorkers] = {};
-    // per-frame launches at 32 lanes: measured ahead of the persistent pair
-    // on batches of 1080p frames, on the config-3 mix and in the config-4
-    // server (lower latency and higher saturated throughput)
+    // per-frame launches: measured ahead of the persistent pair on batches of
+    // 1920x1080 frames, on 64 cameras of mixed sizes and in the server (lower
+    // latency and higher saturated throughput)
     rle_batch_tuning tuning{1, 32, 1, 128, 1, 1};
     int raycast_blocks = 0;
     int resolve_blocks = 0;

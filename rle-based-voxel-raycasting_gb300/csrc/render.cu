@@ -909,6 +909,16 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
     }
 }
 
+// Steps from here that can meet neither a LOD switch nor the end of the ray.
+// z, dz (a power of two) and the switch distances are whole numbers held in
+// floats, exactly below 2^24.
+__device__ __forceinline__ int steps_unchecked(const RayParams& P, const Walk& W) {
+    if (!dda_can_jump(W.d) || !(W.z + W.dz < 16777216.0f)) return 0;
+    const int zi = static_cast<int>(W.z), shift = 31 - __clz(static_cast<int>(W.dz));
+    const int to_switch = W.mapswitch - zi, to_end = min(P.z_far, 16777216) - zi;
+    return to_switch < 0 || to_end < 0 ? 0 : min((to_switch >> shift) + 1, to_end >> shift);
+}
+
 // One chunk of the DDA: lane k's cell is that of step k, from the event of
 // step k and that of the step before (a shuffle from lane k-1; lane 0 takes
 // the last event of the chunk before).  Advances W past the chunk and returns
@@ -928,16 +938,6 @@ __device__ __forceinline__ void merge_chunk(const RayParams& P, const Ray& R, co
 // with the horizon test that drops whole chunks before they are projected
 // (cell_alive) and the word-wise merge, per frame: 1920x1080 438 -> 310 us,
 // 1366x768 with hits 278 -> 225 us, 640x480 152 -> 130 us, 320x240 87 -> 82 us.
-// Steps from here that can meet neither a LOD switch nor the end of the ray.
-// z, dz (a power of two) and the switch distances are whole numbers held in
-// floats, exactly below 2^24.
-__device__ __forceinline__ int steps_unchecked(const RayParams& P, const Walk& W) {
-    if (!dda_can_jump(W.d) || !(W.z + W.dz < 16777216.0f)) return 0;
-    const int zi = static_cast<int>(W.z), shift = 31 - __clz(static_cast<int>(W.dz));
-    const int to_switch = W.mapswitch - zi, to_end = min(P.z_far, 16777216) - zi;
-    return to_switch < 0 || to_end < 0 ? 0 : min((to_switch >> shift) + 1, to_end >> shift);
-}
-
 __device__ __forceinline__ int dda_chunk(const RayParams& P, Walk& W, int k, ChunkStep& st) {
     const float start_dd = W.d.dd_now, start_px = W.d.pnx, start_py = W.d.pny;
     const int start_ix = W.d.index;

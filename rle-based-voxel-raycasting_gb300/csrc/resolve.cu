@@ -85,14 +85,15 @@ __device__ __forceinline__ void resolve_pixel(const ResolveParams& P, int col, i
     }
 }
 
-// Bound by the L1 lines its gathers touch, then by its instructions.  In the up
-// and down fans the pixels of a screen row lie on as many column rays, a line
-// each, and those of a screen column are neighbours on one ray; to the sides it
-// is the other way round.  A warp takes 8x4 pixels, 4 to 8 lines per gather in
-// either (a row of 32: up to 32).  3840x2160 frames: 69 us with the shader's
-// arithmetic as it stands and rows of 128, 63 us with the terms that count
-// (resolve_math.h) and rows of 32, 46 us with 8x4 pixels per warp (4x8: 46, 16x2:
-// 47); 1920x1080: 20, 18, 13 us.
+// Bound by its instructions (issue slots 81% taken at 3840x2160, 74% at
+// 1920x1080), with the L1 close behind (66% and 63%).  In the up and down fans
+// the pixels of a screen row lie on as many column rays, a line each, and those
+// of a screen column are neighbours on one ray; to the sides it is the other way
+// round.  A warp takes 8x4 pixels, 4 to 8 lines per gather in either (a row of
+// 32: up to 32, and the gathers bound it).  3840x2160 frames: 69 us with the
+// shader's arithmetic as it stands and rows of 128, 63 us with the terms that
+// count (resolve_math.h) and rows of 32, 46 us with 8x4 pixels per warp (4x8: 46,
+// 16x2: 47); 1920x1080: 20, 18, 13 us.
 constexpr int kTileX = 32, kTileY = 8;  // pixels of a block
 constexpr int kWarpX = 8, kWarpY = 4;   // pixels of a warp
 static_assert(kWarpX * kWarpY == 32 && kTileX % kWarpX == 0 && kTileY % kWarpY == 0, "tile");
@@ -115,7 +116,9 @@ __global__ void __launch_bounds__(kTileX * kTileY) resolve_kernel(const __grid_c
 // block_start[f] <= b < block_start[f+1] and covers 256 of its pixels.
 constexpr int kResolveBlock = 256;
 
-// Persistent: block i takes pixel blocks i, i + gridDim.x, ... of the batch.
+// Persistent: block i takes pixel blocks i, i + gridDim.x, ... of the batch, in
+// rows: its gathers bound it (L1 80% taken, issue slots 40%; 99 us for eight
+// 1280x720 frames, which as single frames take about half).
 __global__ void __launch_bounds__(kResolveBlock) resolve_batch_kernel(const BatchHeader* __restrict__ hdr,
                                                                       const int* __restrict__ block_start,
                                                                       const ResolveParams* __restrict__ frames) {

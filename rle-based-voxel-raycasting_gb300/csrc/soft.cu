@@ -23,7 +23,10 @@
 // once into shared memory, already divided by 255 and clamped to the frame,
 // then every tap reads shared memory.
 //
-// Bound by instructions and shared-memory reads (33 bilinear taps per pixel).
+// Bound by shared-memory reads and instructions alike (33 bilinear taps per
+// pixel, 1.7 KB of shared memory where it is filtered): on a 1920x1080 frame the
+// L1's data pipe is 68% and the issue slots are 69% taken, at half of the warps'
+// slots.
 // Unpacking RGBA8 at each tap cost 16 IEEE divisions by 255 (the kernel took
 // 332 and 503 us on two 1920x1080 frames); four floats per texel cost one
 // 16-byte read, and the alpha alone, which the circle needs, has a plane of its

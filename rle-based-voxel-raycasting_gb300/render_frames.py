@@ -74,7 +74,8 @@ def main(argv=None) -> int:
     ap.add_argument("--batch", type=int, default=0,
                     help="render the path in batches of this many frames (rle_batch, autotuned) instead")
     ap.add_argument("--batch-lanes", type=int, default=0,
-                    help="with --batch: skip the autotuner, one-ray claims with this many lanes per ray")
+                    help="with --batch: 8, 16 or 32 skips the autotuner (the persistent pair, one-ray claims); "
+                         "the number itself has no effect, a warp casts one ray")
     ap.add_argument("--json", action="store_true", help="one JSON object per frame (or batch) on stdout")
     args = ap.parse_args(argv)
 
@@ -148,8 +149,7 @@ def _batched(rle, torch, scene, info, table, words, rng, view, args) -> int:
         b.set_tuning(1, args.batch_lanes, 1, 128)
     else:
         best, ms = b.autotune(scene, groups[0], repeats=1)
-        msg = (f"autotuned: tile {best.tile_rays} lanes {best.lanes_per_ray} staging {best.staging} "
-               f"per_frame {best.per_frame} ({ms:.3f} ms)")
+        msg = f"autotuned: tile {best.tile_rays} per_frame {best.per_frame} ({ms:.3f} ms)"
         print(msg, file=sys.stderr if args.json else sys.stdout, flush=True)
     for i, g in enumerate(groups):
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

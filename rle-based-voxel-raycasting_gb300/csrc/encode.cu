@@ -833,8 +833,13 @@ rle_status order_behind(Build& B, cudaStream_t stream) {
         cudaGetLastError();
         return RLE_OK;
     }
+    if (e == cudaSuccess) e = cudaStreamQuery(stream);
+    if (e == cudaSuccess) return RLE_OK;  // nothing queued (the usual case)
     cudaEvent_t done = nullptr;
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    if (e == cudaErrorNotReady) {
+        cudaGetLastError();
+        e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+    }
     if (e == cudaSuccess) e = cudaEventRecord(done, stream);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(B.stream, done, 0);
     if (done) cudaEventDestroy(done);
